@@ -2,16 +2,15 @@
 // particle substep (integration, particle-shape and particle-particle
 // contacts, springs, position corrections).
 //
-// Layout: particles are SoA float3 rows ([P,3]); every kernel runs one thread
-// per particle.  Each particle GATHERS its corrections (its own soft contacts,
+// Layout: particles are SoA float3 rows ([P,3]).  Each particle GATHERS its corrections (its own soft contacts,
 // its neighbours, its springs) in a fixed order and writes its delta once, in
 // place of the reference's per-constraint atomic scatter: no atomics on the
 // data path and the same bits on every run.
 //
-// Particle-particle neighbours come from two hashed cell tables, rebuilt from
-// the positions each iteration reads: the apply kernel of iteration i inserts
-// every particle into table (i+1)&1 as it writes its new position, and the
-// constraint kernel of iteration i clears table (i+1)&1 before that.
+// Particle-particle neighbours come from a hashed cell grid, rebuilt every
+// iteration from the positions it reads (struct Grid below): the apply kernel
+// of iteration i counts every particle into its bucket as it writes its new
+// position, and two small kernels put the particles' entries in bucket order.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -225,21 +224,98 @@ __global__ void __launch_bounds__(kScanThreads) soft_write_kernel(NbParticleDesc
 }
 
 // ---------------------------------------------------------------- substep
+// Neighbour search.  Cells have the size of the largest contact distance; a cell's bucket is
+// (cx + cy K1 + cz K2) mod M, so cells that follow each other in x are buckets that follow each other,
+// and the up to 3 cells of one (cy, cz) row around a particle are one run of the particles in bucket
+// order: 9 runs of about 14 particles in place of 27 chains.  Two forms:
+//   sorted: per iteration the particles are counted into the buckets (integrate / apply), the buckets
+//           get their ranges (particle_ranges_kernel) and the particles' entries are written there
+//           (particle_scatter_kernel).  An entry is 8 bytes: the position within 4 cells, 10 bits per
+//           axis, and the particle -- enough to reject five of six candidates with one load.
+//   lists:  linked lists per bucket (head / next), for scratch too small for the sorted form.
 struct Grid {
-    int32_t* head;  // [2*size]
-    int32_t* next;  // [P]
-    uint32_t mask;
+    int32_t* head;   // lists: [2][M] first particle of a bucket, -1 empty
+    int32_t* next;   // lists: [P] next particle of the same bucket
+    int2* range;     // sorted: [M] first and last + 1 entry of a bucket
+    int2* entry;     // sorted: [P] (packed position, particle) in bucket order
+    int32_t* count;  // sorted: [M] particles of a bucket; all zero outside counting .. scatter
+    int32_t* cursor; // sorted: [1] entries handed out so far; the active particles once all are
+    uint32_t mask;   // M - 1
     float inv_h;
-    bool on;
+    bool on, sorted;
 };
+
+constexpr int kRangeBuckets = 1024;  // buckets whose ranges one block lays out contiguously
+constexpr int kMinSorted = 8;        // fewest buckets of the sorted form: a row of 5 cells never wraps onto itself
 
 NB_D int cell_of(float x, float inv_h) { return (int)floorf(x * inv_h); }
 NB_D uint32_t cell_hash(int cx, int cy, int cz, uint32_t mask) {
-    return ((uint32_t)cx * 73856093u ^ (uint32_t)cy * 19349663u ^ (uint32_t)cz * 83492791u) & mask;
+    return ((uint32_t)cx + (uint32_t)cy * 0x9E3779B1u + (uint32_t)cz * 0x85EBCA77u) & mask;
+}
+// position within 4 cells in 1/256 cells
+NB_D uint32_t pack_axis(float x, float inv_h) {
+    const float t = x * inv_h, c = floorf(t);
+    const int f = (int)((t - c) * 256.0f);
+    return (((uint32_t)(int)c & 3u) << 8) | (uint32_t)min(max(f, 0), 255);
+}
+NB_D uint32_t pack_pos(V3 x, float inv_h) {
+    return pack_axis(x.x, inv_h) | (pack_axis(x.y, inv_h) << 10) | (pack_axis(x.z, inv_h) << 20);
 }
 NB_D void grid_insert(const Grid& g, int table, int p, V3 x) {
     const uint32_t b = cell_hash(cell_of(x.x, g.inv_h), cell_of(x.y, g.inv_h), cell_of(x.z, g.inv_h), g.mask);
-    g.next[p] = atomicExch(&g.head[(size_t)table * (g.mask + 1u) + b], p);
+    if (g.sorted) atomicAdd(&g.count[b], 1);
+    else g.next[p] = atomicExch(&g.head[(size_t)table * (g.mask + 1u) + b], p);
+}
+
+// Ranges of kRangeBuckets buckets per block: an exclusive scan of their counts from a base taken off the
+// cursor.  Which block comes first decides only where its entries lie; within the block they are in
+// bucket order.
+__global__ void __launch_bounds__(kThreads) particle_ranges_kernel(Grid g) {
+    __shared__ int s_warp[kThreads / 32];
+    __shared__ int s_base;
+    constexpr int kPer = kRangeBuckets / kThreads;
+    const uint32_t b0 = blockIdx.x * kRangeBuckets + threadIdx.x * kPer;
+    int c[kPer], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        c[k] = b0 + k <= g.mask ? g.count[b0 + k] : 0;
+        sum += c[k];
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int run = 0;
+        for (int w = 0; w < kThreads / 32; ++w) {
+            const int v = s_warp[w];
+            s_warp[w] = run;
+            run += v;
+        }
+        s_base = run > 0 ? atomicAdd(g.cursor, run) : 0;
+    }
+    __syncthreads();
+    int at = s_base + s_warp[warp] + x - sum;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        if (b0 + k <= g.mask) g.range[b0 + k] = make_int2(at, at + c[k]);
+        at += c[k];
+    }
+}
+
+// The particles' entries into their buckets' ranges; leaves every count at zero.
+__global__ void __launch_bounds__(kThreads) particle_scatter_kernel(NbParticleDesc pd, const float* xq, Grid g) {
+    const int p = blockIdx.x * kThreads + threadIdx.x;
+    if (p >= pd.particle_count || !active(pd, p)) return;
+    const V3 x = ld3(xq, p);
+    const uint32_t b = cell_hash(cell_of(x.x, g.inv_h), cell_of(x.y, g.inv_h), cell_of(x.z, g.inv_h), g.mask);
+    const int at = g.range[b].x + atomicSub(&g.count[b], 1) - 1;
+    g.entry[at] = make_int2((int)pack_pos(x, g.inv_h), p);
 }
 
 // integrate_particles (newton/_src/solvers/solver.py:11-47): semi-implicit Euler, gravity on
@@ -248,6 +324,7 @@ __global__ void __launch_bounds__(kThreads) particle_integrate_kernel(NbParticle
                                                                       float dt, Grid g) {
     const int p = blockIdx.x * kThreads + threadIdx.x;
     if (p >= pd.particle_count) return;
+    if (p == 0 && g.sorted) g.cursor[0] = 0;
     const V3 x0 = ld3(io.particle_q, p);
     const V3 v0 = ld3(io.particle_qd, p);
     if (!active(pd, p)) {
@@ -271,184 +348,299 @@ __global__ void __launch_bounds__(kThreads) particle_integrate_kernel(NbParticle
 
 // The corrections of one particle in one iteration: soft contacts (kernels.py:114-222, static
 // shapes), particle neighbours (kernels.py:225-289) and springs (kernels.py:292-356), summed in
-// that order.  kGroup lanes serve one particle: they split its neighbour cells between them (the
-// cell-list walks are chains of dependent loads) and each computes the contribution of the
-// neighbours it accepts; the group's first lane sorts them by neighbour index and sums them in that
-// order, then adds the soft contacts and springs.  Which lane computes a contribution does not change
-// its bits, so the result equals a sequential sum in ascending neighbour index.  The kernel also
-// clears the cell table the following apply fills.
-#ifndef NB_PARTICLE_GROUP
-#define NB_PARTICLE_GROUP 8
-#endif
-constexpr int kGroup = NB_PARTICLE_GROUP;  // lanes per particle: 2, 4, 8 or 16
-static_assert(kGroup >= 2 && kGroup <= 16 && (kGroup & (kGroup - 1)) == 0, "lanes per particle");
+// that order.  kGroup lanes serve one particle: they filter the candidates of its cell rows by the packed
+// positions, kept ones go to a list in shared memory, each lane tests its share of the list exactly and
+// then computes the contributions of its share of the contacting ones (and of the springs); every lane
+// sums them in ascending neighbour (spring) index.  Which lane computes a contribution does not change its
+// bits, so the result equals a sequential sum in that order.
+// Bound by the latency of the dependent loads and, at size, by instructions, so the steps are few and
+// wide: one row lookup per lane, candidates in runs of 32, all arrays of a kept candidate at once; the
+// sorted form takes the particles in bucket order, so that a block's particles share their candidates in
+// L1.  Measured at 110,002 particles (54 candidates, 4 contacts each on average; 8 iterations, per
+// substep) with 4 / 8 / 16 / 32 lanes: 1369 / 990 / 967 / 1440 us; at 3,010 particles (4 iterations):
+// 286 / 205 / 150 / 147 us.  Linked lists of the cells, whose candidates are one dependent load after
+// another, with one lane sorting and summing for its group of 8, took 2215 and 240 us.
+constexpr int kGroup = 16;                 // lanes per particle
 constexpr int kSlots = kThreads / kGroup;  // particles per block
+constexpr int kAhead = 2;                  // candidate loads a lane has in flight
+constexpr int kMaybe = 2 * kAhead * kGroup;
 
-__global__ void __launch_bounds__(kThreads) particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io,
-                                                                        NbSoftContacts sc, int has_sc, float dt,
-                                                                        float relaxation, Grid g, int table) {
-    __shared__ int s_n[kSlots];
-    __shared__ int s_j[kSlots][NB_PARTICLE_MAX_NEIGHBORS];
-    __shared__ float s_c[kSlots][NB_PARTICLE_MAX_NEIGHBORS][3];
+// A group's scratch: the candidates' runs and list, then (in the same place) the contributions.
+struct GroupScratch {
+    // runs of entries (a row may be cut in two): entry minus running index, running index past the run,
+    // low cell bits of the row where the packed position has them, row
+    union {
+        struct {
+            int4 seg[2 * kGroup];
+            int maybe[kMaybe];                         // candidates to be tested exactly
+        };
+        float c[NB_PARTICLE_MAX_NEIGHBORS][3];     // the accepted neighbours' contributions, in ascending index
+    };
+    int j[NB_PARTICLE_MAX_NEIGHBORS];              // accepted neighbours
+    int nm, n;                                     // candidates listed, neighbours accepted
+};
+
+template <bool kSorted>
+__global__ void __launch_bounds__(kThreads, 4)
+particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io, NbSoftContacts sc, int has_sc, float dt,
+                            float relaxation, Grid g, int table) {
+    __shared__ GroupScratch s_group[kSlots];
     const int tid = blockIdx.x * kThreads + threadIdx.x;
-    if (g.on) {
+    if (!kSorted && g.on) {
+        // clears the lists the following apply fills
         int32_t* other = g.head + (size_t)(table ^ 1) * (g.mask + 1u);
         for (uint32_t t = tid; t <= g.mask; t += gridDim.x * kThreads) other[t] = -1;
     }
     const int lane = threadIdx.x & (kGroup - 1);
-    const int slot = threadIdx.x / kGroup;
     const unsigned gmask = ((1u << kGroup) - 1u) << (threadIdx.x & 31 & ~(kGroup - 1));
-    const int i = blockIdx.x * kSlots + slot;
-    const bool valid = i < pd.particle_count;
-    const bool act = valid && active(pd, i);
+    GroupScratch& G = s_group[threadIdx.x / kGroup];
+    int i = blockIdx.x * kSlots + threadIdx.x / kGroup;
+    if constexpr (kSorted) {
+        if (i >= g.cursor[0]) return;  // the whole group; inactive particles have no entry and need no delta
+        i = g.entry[i].y;
+    } else {
+        if (i >= pd.particle_count || !active(pd, i)) return;
+    }
     const float* xq = io.particle_q_out;
     const float* vq = io.particle_qd_out;
-    if (lane == 0) s_n[slot] = 0;
+    const V3 x = ld3(xq, i), v = ld3(vq, i);
+    const float w1 = pd.particle_inv_mass[i], radius = pd.particle_radius[i];
+    const int spring_lo = pd.spring_count > 0 ? pd.particle_spring_start[i] : 0;
+    const int spring_hi = pd.spring_count > 0 ? pd.particle_spring_start[i + 1] : 0;
+    const int soft_lo = has_sc ? sc.particle_start[i] : 0;
+    const int soft_hi = has_sc ? min(sc.particle_start[i + 1], min(sc.max, sc.count[0])) : 0;
+    if (lane == 0) G.nm = G.n = 0;
     __syncwarp(gmask);
-    V3 x = V3{0.0f, 0.0f, 0.0f}, v = x;
-    float w1 = 0.0f, radius = 0.0f;
-    if (valid) {
-        x = ld3(xq, i);
-        v = ld3(vq, i);
-        w1 = pd.particle_inv_mass[i];
-        radius = pd.particle_radius[i];
-    }
 
-    if (act && g.on) {
+    if (g.on) {
         const float reach = (radius + pd.particle_max_radius + pd.particle_cohesion) * 1.001f + 1.0e-6f;
         // the reach is at most ~1 cell (cell size 2 * max radius + cohesion), so a span of 3 cells per axis;
         // the cap keeps the loops bounded whatever the scale
         const int x0 = cell_of(x.x - reach, g.inv_h), x1 = min(cell_of(x.x + reach, g.inv_h), x0 + 4);
         const int y0 = cell_of(x.y - reach, g.inv_h), y1 = min(cell_of(x.y + reach, g.inv_h), y0 + 4);
         const int z0 = cell_of(x.z - reach, g.inv_h), z1 = min(cell_of(x.z + reach, g.inv_h), z0 + 4);
-        const int nx = x1 - x0 + 1, ny = y1 - y0 + 1, ncell = nx * ny * (z1 - z0 + 1);
-        const int32_t* head = g.head + (size_t)table * (g.mask + 1u);
-        bool overflow = false;
-        for (int c = lane; c < ncell; c += kGroup) {
-            const int cx = x0 + c % nx, cy = y0 + (c / nx) % ny, cz = z0 + c / (nx * ny);
-            for (int j = head[cell_hash(cx, cy, cz, g.mask)]; j >= 0; j = g.next[j]) {
-                if (j == i) continue;
-                const V3 xj = ld3(xq, j);
-                // each particle sits in one cell: skip other cells hashed to this bucket
-                if (cell_of(xj.x, g.inv_h) != cx || cell_of(xj.y, g.inv_h) != cy || cell_of(xj.z, g.inv_h) != cz)
-                    continue;
-                if (!active(pd, j)) continue;
-                V3 n = sub(x, xj);
-                const float d = length(n);
-                const float err = d - radius - pd.particle_radius[j];
-                const float denom = w1 + pd.particle_inv_mass[j];
-                if (!(err <= pd.particle_cohesion && denom > 0.0f)) continue;
-                const int at = atomicAdd(&s_n[slot], 1);
-                if (at >= NB_PARTICLE_MAX_NEIGHBORS) {
-                    overflow = true;
-                    continue;
-                }
-                n = divs(n, d);
-                const V3 vrel = sub(v, ld3(vq, j));
-                const float lambda_n = err;
-                const V3 delta_n = mul(n, lambda_n);
-                const float vn = dot(n, vrel);
-                const V3 vt = sub(vrel, mul(n, vn));
-                const float lambda_f = fmaxw(pd.particle_mu * lambda_n, -length(vt) * dt);
-                const V3 delta_f = mul(normalize(vt), lambda_f);
-                const V3 contrib = divs(sub(delta_f, delta_n), denom);
-                s_j[slot][at] = j;
-                s_c[slot][at][0] = contrib.x;
-                s_c[slot][at][1] = contrib.y;
-                s_c[slot][at][2] = contrib.z;
+        // tests candidate j exactly
+        auto consider = [&](int j) {
+            const V3 xj = ld3(xq, j);
+            const float rj = pd.particle_radius[j], wj = pd.particle_inv_mass[j];
+            const int cx = cell_of(xj.x, g.inv_h), cy = cell_of(xj.y, g.inv_h), cz = cell_of(xj.z, g.inv_h);
+            const V3 n = sub(x, xj);
+            const float d = length(n);
+            const float err = d - radius - rj;
+            const float denom = w1 + wj;
+            if (cx >= x0 && cx <= x1 && cy >= y0 && cy <= y1 && cz >= z0 && cz <= z1 && err <= pd.particle_cohesion &&
+                denom > 0.0f) {
+                const int at = atomicAdd(&G.n, 1);
+                if (at < NB_PARTICLE_MAX_NEIGHBORS) G.j[at] = j;
             }
+        };
+        const int ny = y1 - y0 + 1, rows = ny * (z1 - z0 + 1);
+        if constexpr (kSorted) {
+            // squared reach in the packed positions' units: a packed difference is off by less than 1 per
+            // axis, and by the rounding of x * inv_h far from the origin; past half the packed period
+            // nothing is rejected
+            const float far = fmaxf(fabsf(x.x), fmaxf(fabsf(x.y), fabsf(x.z))) + reach;
+            const float ru = (reach * 256.0f + far * 1.0e-4f) * g.inv_h + 2.0f;
+            const int r2 = ru < 500.0f ? (int)(ru * ru) + 1 : 0x7fffffff;
+            const uint32_t mine = pack_pos(x, g.inv_h);
+            const uint32_t bm = min((uint32_t)kRangeBuckets - 1u, g.mask);
+            // a candidate belongs to the row it is met in (rows may share buckets): by its cells' low two
+            // bits, which tell up to 4 rows apart, or by its cells where there are 5
+            const bool wide = ny > 4 || rows > 4 * ny;
+            for (int r0 = 0; r0 < rows; r0 += kGroup) {
+                // each lane looks one row up: one run of entries, or two where the row leaves its block
+                const int r = r0 + lane;
+                int beg = 0, len = 0, beg2 = 0, tot = 0;
+                uint32_t key = 0u;
+                if (r < rows) {
+                    const int rz = (int)__fdividef((float)r + 0.5f, (float)ny);  // r / ny: both below 32
+                    const int cy = y0 + r - rz * ny, cz = z0 + rz;
+                    key = (((uint32_t)cy & 3u) << 18) | (((uint32_t)cz & 3u) << 28);
+                    const uint32_t b = cell_hash(x0, cy, cz, g.mask);
+                    const uint32_t e = b + (uint32_t)(x1 - x0), cut = b | bm;
+                    beg = g.range[b].x;
+                    len = g.range[min(e, cut)].y - beg;
+                    tot = len;
+                    if (e > cut) {
+                        beg2 = g.range[(cut + 1u) & g.mask].x;
+                        tot += g.range[e & g.mask].y - beg2;
+                    }
+                }
+                int run = tot;
+#pragma unroll
+                for (int o = 1; o < kGroup; o <<= 1) {
+                    const int y = __shfl_up_sync(gmask, run, o, kGroup);
+                    if (lane >= o) run += y;
+                }
+                const int total = __shfl_sync(gmask, run, kGroup - 1, kGroup);
+                run -= tot;
+                G.seg[2 * lane] = make_int4(beg - run, run + len, (int)key, r);
+                G.seg[2 * lane + 1] = make_int4(beg2 - run - len, run + tot, (int)key, r);
+                __syncwarp(gmask);
+                int q = 0;
+                int4 seg = G.seg[0];
+                for (int base = 0; base < total; base += kAhead * kGroup) {
+                    int2 en[kAhead];
+                    uint32_t row_key[kAhead];
+#pragma unroll
+                    for (int u = 0; u < kAhead; ++u) {
+                        const int a = base + u * kGroup + lane;
+                        en[u].y = i;  // none
+                        if (a < total) {
+                            while (a >= seg.y) seg = G.seg[++q];
+                            en[u] = g.entry[seg.x + a];
+                            row_key[u] = (uint32_t)seg.z;
+                            if (wide) {
+                                const V3 xj = ld3(xq, en[u].y);
+                                const int rz = seg.w / ny;
+                                if (cell_of(xj.y, g.inv_h) != y0 + seg.w - rz * ny ||
+                                    cell_of(xj.z, g.inv_h) != z0 + rz)
+                                    en[u].y = i;
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < kAhead; ++u) {
+                        const uint32_t w = (uint32_t)en[u].x;
+                        const int dx = (int)((w - mine) << 22) >> 22;
+                        const int dy = (int)(((w >> 10) - (mine >> 10)) << 22) >> 22;
+                        const int dz = (int)(((w >> 20) - (mine >> 20)) << 22) >> 22;
+                        if (en[u].y != i && ((w ^ row_key[u]) & 0x300C0000u) == 0u && dx * dx + dy * dy + dz * dz <= r2)
+                            G.maybe[atomicAdd(&G.nm, 1)] = en[u].y;
+                    }
+                    __syncwarp(gmask);
+                    // the list is tested when another round might not fit, and at the end
+                    const int nm = G.nm;
+                    if (nm > kMaybe - kAhead * kGroup || base + kAhead * kGroup >= total) {
+                        for (int a = lane; a < nm; a += kGroup) consider(G.maybe[a]);
+                        __syncwarp(gmask);
+                        if (lane == 0) G.nm = 0;
+                        __syncwarp(gmask);
+                    }
+                }
+            }
+        } else {
+            const int nx = x1 - x0 + 1, ncell = nx * rows;
+            const int32_t* head = g.head + (size_t)table * (g.mask + 1u);
+            for (int c = lane; c < ncell; c += kGroup) {
+                const int cx = x0 + c % nx, cy = y0 + (c / nx) % ny, cz = z0 + c / (nx * ny);
+                for (int j = head[cell_hash(cx, cy, cz, g.mask)]; j >= 0; j = g.next[j]) {
+                    if (j == i) continue;
+                    const V3 xj = ld3(xq, j);
+                    // each particle sits in one cell: skip other cells hashed to this bucket
+                    if (cell_of(xj.x, g.inv_h) == cx && cell_of(xj.y, g.inv_h) == cy && cell_of(xj.z, g.inv_h) == cz)
+                        consider(j);
+                }
+            }
+            __syncwarp(gmask);
         }
-        if (overflow) atomicOr(io.status, NB_STATUS_NEIGHBOR_OVERFLOW);
+        if (lane == 0 && G.n > NB_PARTICLE_MAX_NEIGHBORS) atomicOr(io.status, NB_STATUS_NEIGHBOR_OVERFLOW);
+        const int count = min(G.n, NB_PARTICLE_MAX_NEIGHBORS);
+        for (int a = lane; a < count; a += kGroup) {
+            const int j = G.j[a];
+            const V3 vj = ld3(vq, j);
+            V3 n = sub(x, ld3(xq, j));
+            const float d = length(n);
+            const float err = d - radius - pd.particle_radius[j];
+            const float denom = w1 + pd.particle_inv_mass[j];
+            int rank = 0;
+            for (int b = 0; b < count; ++b) rank += G.j[b] < j ? 1 : 0;
+            n = divs(n, d);
+            const V3 vrel = sub(v, vj);
+            const float lambda_n = err;
+            const V3 delta_n = mul(n, lambda_n);
+            const float vn = dot(n, vrel);
+            const V3 vt = sub(vrel, mul(n, vn));
+            const float lambda_f = fmaxw(pd.particle_mu * lambda_n, -length(vt) * dt);
+            const V3 delta_f = mul(normalize(vt), lambda_f);
+            const V3 contrib = divs(sub(delta_f, delta_n), denom);
+            G.c[rank][0] = contrib.x;
+            G.c[rank][1] = contrib.y;
+            G.c[rank][2] = contrib.z;
+        }
+        __syncwarp(gmask);
     }
-    __syncwarp(gmask);
-    if (lane != 0 || !valid) return;
 
     V3 delta = V3{0.0f, 0.0f, 0.0f};
-    if (act && has_sc) {
-        const int lim = min(sc.max, sc.count[0]);
-        const int hi = min(sc.particle_start[i + 1], lim);
-        for (int k = sc.particle_start[i]; k < hi; ++k) {
-            const int s = sc.shape[k];
-            if (pd.shape_body[s] >= 0) {
-                atomicOr(io.status, NB_STATUS_PARTICLE_BODY_CONTACT);
-                continue;
-            }
-            // static shape: identity body transform, zero body velocity
-            const TF X_wb = tf_identity();
-            const V3 bx = tf_point(X_wb, ld3(sc.body_pos, k));
-            const V3 r = sub(bx, tf_point(X_wb, V3{0.0f, 0.0f, 0.0f}));
-            const V3 n = ld3(sc.normal, k);
-            const float c = dot(n, sub(x, bx)) - radius;
-            if (c > pd.particle_adhesion) continue;
-            const float mu = 0.5f * (pd.soft_contact_mu + pd.shape_mu[s]);
-            const V3 body_w = V3{0.0f, 0.0f, 0.0f}, body_v = V3{0.0f, 0.0f, 0.0f};
-            const V3 bv = add(add(body_v, cross(body_w, r)), tf_vector(X_wb, ld3(sc.body_vel, k)));
-            const V3 vr = sub(v, bv);
-            const float lambda_n = c;
-            const V3 delta_n = mul(n, lambda_n);
-            const float vn = dot(n, vr);
-            const V3 vt = sub(vr, mul(n, vn));
-            const float denom = w1 + 0.0f;
-            if (denom == 0.0f) continue;
-            const float lambda_f = fmaxw(mu * lambda_n, -length(vt) * dt);
-            const V3 delta_f = mul(normalize(vt), lambda_f);
-            const V3 delta_total = mul(divs(sub(delta_f, delta_n), denom), relaxation);
-            delta = add(delta, smul(w1, delta_total));
+    for (int k = soft_lo; k < soft_hi; ++k) {
+        const int s = sc.shape[k];
+        // static shape: identity body transform, zero body velocity
+        const TF X_wb = tf_identity();
+        const V3 bx = tf_point(X_wb, ld3(sc.body_pos, k));
+        const V3 r = sub(bx, tf_point(X_wb, V3{0.0f, 0.0f, 0.0f}));
+        const V3 n = ld3(sc.normal, k);
+        const V3 body_vel = ld3(sc.body_vel, k);
+        const float mu = 0.5f * (pd.soft_contact_mu + pd.shape_mu[s]);
+        if (pd.shape_body[s] >= 0) {
+            if (lane == 0) atomicOr(io.status, NB_STATUS_PARTICLE_BODY_CONTACT);
+            continue;
         }
+        const float c = dot(n, sub(x, bx)) - radius;
+        if (c > pd.particle_adhesion) continue;
+        const V3 body_w = V3{0.0f, 0.0f, 0.0f}, body_v = V3{0.0f, 0.0f, 0.0f};
+        const V3 bv = add(add(body_v, cross(body_w, r)), tf_vector(X_wb, body_vel));
+        const V3 vr = sub(v, bv);
+        const float lambda_n = c;
+        const V3 delta_n = mul(n, lambda_n);
+        const float vn = dot(n, vr);
+        const V3 vt = sub(vr, mul(n, vn));
+        const float denom = w1 + 0.0f;
+        if (denom == 0.0f) continue;
+        const float lambda_f = fmaxw(mu * lambda_n, -length(vt) * dt);
+        const V3 delta_f = mul(normalize(vt), lambda_f);
+        const V3 delta_total = mul(divs(sub(delta_f, delta_n), denom), relaxation);
+        delta = add(delta, smul(w1, delta_total));
     }
 
-    if (act && g.on) {
-        // neighbours in ascending index (insertion sort of the group's accepted list)
-        const int count = min(s_n[slot], NB_PARTICLE_MAX_NEIGHBORS);
-        int* js = s_j[slot];
-        float(*cs)[3] = s_c[slot];
-        for (int a = 1; a < count; ++a) {
-            const int j = js[a];
-            const float c0 = cs[a][0], c1 = cs[a][1], c2 = cs[a][2];
-            int b = a;
-            while (b > 0 && js[b - 1] > j) {
-                js[b] = js[b - 1];
-                cs[b][0] = cs[b - 1][0];
-                cs[b][1] = cs[b - 1][1];
-                cs[b][2] = cs[b - 1][2];
-                --b;
-            }
-            js[b] = j;
-            cs[b][0] = c0;
-            cs[b][1] = c1;
-            cs[b][2] = c2;
-        }
+    if (g.on) {
+        const int count = min(G.n, NB_PARTICLE_MAX_NEIGHBORS);
         V3 dpp = V3{0.0f, 0.0f, 0.0f};
-        for (int k = 0; k < count; ++k) dpp = add(dpp, V3{cs[k][0], cs[k][1], cs[k][2]});
+        for (int k = 0; k < count; ++k) {
+            const float* c = G.c[k];
+            dpp = add(dpp, V3{c[0], c[1], c[2]});
+        }
         delta = add(delta, mul(mul(dpp, w1), relaxation));
     }
 
-    if (pd.spring_count > 0) {
-        const int s_hi = pd.particle_spring_start[i + 1];
-        for (int k = pd.particle_spring_start[i]; k < s_hi; ++k) {
-            const int s = pd.particle_spring_list[k];
-            const int a = pd.spring_indices[2 * s], b = pd.spring_indices[2 * s + 1];
-            const float ke = pd.spring_stiffness[s], kd = pd.spring_damping[s], rest = pd.spring_rest_length[s];
-            const V3 xij = sub(ld3(xq, a), ld3(xq, b));
-            const V3 vij = sub(ld3(vq, a), ld3(vq, b));
-            const float l = length(xij);
-            if (l == 0.0f) continue;
-            const V3 n = divs(xij, l);
-            const float c = l - rest;
-            const float wi = pd.particle_inv_mass[a], wj = pd.particle_inv_mass[b];
-            const float denom = wi + wj;
-            if (denom <= 0.0f || ke <= 0.0f || kd < 0.0f) continue;
-            const float alpha = 1.0f / (ke * dt * dt);
-            const float gamma = kd / (ke * dt);
-            const float grad_c_dot_v = dt * dot(n, vij);
-            const float lambda_prev = 0.0f;  // the solver zeroes the spring multipliers every iteration
-            const float dlambda =
-                -1.0f * (c + alpha * lambda_prev + gamma * grad_c_dot_v) / ((1.0f + gamma) * denom + alpha);
-            if (i == a) delta = add(delta, mul(n, wi * dlambda));
-            if (i == b) delta = add(delta, mul(smul(-1.0f, n), wj * dlambda));
+    {
+        const int s_hi = spring_hi;
+        for (int k0 = spring_lo; k0 < s_hi; k0 += kGroup) {
+            // each lane one spring: its direction (toward increasing delta of particle i) and magnitude
+            V3 dir = V3{0.0f, 0.0f, 0.0f};
+            float mag = 0.0f;
+            bool on = false;
+            if (k0 + lane < s_hi) {
+                const int s = pd.particle_spring_list[k0 + lane];
+                const int a = pd.spring_indices[2 * s], b = pd.spring_indices[2 * s + 1];
+                const float ke = pd.spring_stiffness[s], kd = pd.spring_damping[s], rest = pd.spring_rest_length[s];
+                const V3 xij = sub(ld3(xq, a), ld3(xq, b));
+                const V3 vij = sub(ld3(vq, a), ld3(vq, b));
+                const float l = length(xij);
+                const V3 n = divs(xij, l);
+                const float c = l - rest;
+                const float wi = pd.particle_inv_mass[a], wj = pd.particle_inv_mass[b];
+                const float denom = wi + wj;
+                on = l != 0.0f && !(denom <= 0.0f || ke <= 0.0f || kd < 0.0f);
+                const float alpha = 1.0f / (ke * dt * dt);
+                const float gamma = kd / (ke * dt);
+                const float grad_c_dot_v = dt * dot(n, vij);
+                const float lambda_prev = 0.0f;  // the solver zeroes the spring multipliers every iteration
+                const float dlambda =
+                    -1.0f * (c + alpha * lambda_prev + gamma * grad_c_dot_v) / ((1.0f + gamma) * denom + alpha);
+                // a spring's ends are two particles (l != 0)
+                dir = i == a ? n : smul(-1.0f, n);
+                mag = i == a ? wi * dlambda : wj * dlambda;
+            }
+            const int nk = min(s_hi - k0, kGroup);
+            for (int k = 0; k < nk; ++k) {
+                const V3 kd3 = V3{__shfl_sync(gmask, dir.x, k, kGroup), __shfl_sync(gmask, dir.y, k, kGroup),
+                                  __shfl_sync(gmask, dir.z, k, kGroup)};
+                const float km = __shfl_sync(gmask, mag, k, kGroup);
+                if (__shfl_sync(gmask, on ? 1 : 0, k, kGroup)) delta = add(delta, mul(kd3, km));
+            }
         }
     }
-    st3(io.delta, i, delta);
+    if (lane == 0) st3(io.delta, i, delta);
 }
 
 NB_D float det3(const M33& m) {
@@ -471,59 +663,132 @@ NB_D M33 from_cols(V3 a, V3 b, V3 c) {
 }
 NB_D V3 col(const M33& m, int c) { return V3{m.m[0][c], m.m[1][c], m.m[2][c]}; }
 
-// Tetrahedra of one particle (solve_tetrahedra, kernels.py:459-628): per element a stretch term
-// (trace(F^T F) - 3) and a volume term (det F - 1), each a compliant constraint with compliance
+// Lanes that share one particle's elements in particle_bending_kernel: an inner cloth particle has 4
+// bending edges, so each lane computes one, and the lanes then add all of them in ascending element index.
+constexpr int kElemGroup = 4;
+constexpr int kElemSlots = kThreads / kElemGroup;  // particles per block
+
+// One lane's terms: up to 4 vertices' corrections grad * mag (bit r of `on` when vertex r is the
+// particle and the term is live).
+struct ElemTerms {
+    V3 grad[4];
+    float mag[4];
+    unsigned on;
+};
+
+// The lanes' terms added to every lane's delta, lane after lane, vertex after vertex.
+NB_D V3 add_terms(const ElemTerms& t, unsigned gmask, int lanes, V3 delta) {
+    for (int k = 0; k < lanes; ++k) {
+        const unsigned on = __shfl_sync(gmask, t.on, k, kElemGroup);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            if (!((on >> r) & 1u)) continue;
+            const V3 gr = V3{__shfl_sync(gmask, t.grad[r].x, k, kElemGroup),
+                             __shfl_sync(gmask, t.grad[r].y, k, kElemGroup),
+                             __shfl_sync(gmask, t.grad[r].z, k, kElemGroup)};
+            delta = add(delta, mul(gr, __shfl_sync(gmask, t.mag[r], k, kElemGroup)));
+        }
+    }
+    return delta;
+}
+
+// One bending edge (bending_constraint, kernels.py:358-457) as seen by particle i.
+NB_D void edge_terms(const NbParticleDesc& pd, const float* xq, const float* vq, int i, int e, float dt,
+                     ElemTerms& t) {
+    t.on = 0u;
+    const int* ix = pd.edge_indices + 4 * e;
+    const float ke = pd.edge_bending_properties[2 * e], kd = pd.edge_bending_properties[2 * e + 1];
+    const V3 x1 = ld3(xq, ix[0]), x2 = ld3(xq, ix[1]), x3 = ld3(xq, ix[2]), x4 = ld3(xq, ix[3]);
+    const float w[4] = {pd.particle_inv_mass[ix[0]], pd.particle_inv_mass[ix[1]], pd.particle_inv_mass[ix[2]],
+                        pd.particle_inv_mass[ix[3]]};
+    const V3 n1 = cross(sub(x3, x1), sub(x4, x1));
+    const V3 n2 = cross(sub(x4, x2), sub(x3, x2));
+    const V3 ev = sub(x4, x3);
+    const float n1_length = length(n1), n2_length = length(n2), e_length = length(ev);
+    if (n1_length < 1.0e-6f || n2_length < 1.0e-6f || e_length < 1.0e-6f) return;
+    const V3 n1_hat = divs(n1, n1_length), n2_hat = divs(n2, n2_length), e_hat = divs(ev, e_length);
+    const float cos_theta = dot(n1_hat, n2_hat);
+    const float sin_theta = dot(cross(n1_hat, n2_hat), e_hat);
+    const float c = nb_atan2(sin_theta, cos_theta) - pd.edge_rest_angle[e];
+    V3* grad = t.grad;
+    grad[0] = mul(neg(n1_hat), e_length);
+    grad[1] = mul(neg(n2_hat), e_length);
+    grad[2] = sub(mul(neg(n1_hat), dot(sub(x1, x4), e_hat)), mul(n2_hat, dot(sub(x2, x4), e_hat)));
+    grad[3] = sub(mul(neg(n1_hat), dot(sub(x3, x1), e_hat)), mul(n2_hat, dot(sub(x3, x2), e_hat)));
+    const float denominator = w[0] * length_sq(grad[0]) + w[1] * length_sq(grad[1]) + w[2] * length_sq(grad[2]) +
+                              w[3] * length_sq(grad[3]);
+    if (denominator <= 0.0f || ke <= 0.0f || kd < 0.0f) return;
+    const float alpha = 1.0f / (ke * dt * dt);
+    const float gamma = kd / (ke * dt);
+    const float grad_dot_v = dt * (dot(grad[0], ld3(vq, ix[0])) + dot(grad[1], ld3(vq, ix[1])) +
+                                   dot(grad[2], ld3(vq, ix[2])) + dot(grad[3], ld3(vq, ix[3])));
+    const float lambda_prev = 0.0f;
+    const float dlambda =
+        -1.0f * (c + alpha * lambda_prev + gamma * grad_dot_v) / ((1.0f + gamma) * denominator + alpha);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        t.mag[r] = w[r] * dlambda;
+        if (ix[r] == i) t.on |= 1u << r;
+    }
+}
+
+// One term of a tetrahedron (solve_tetrahedra, kernels.py:459-628) as seen by particle i: term 0 the
+// stretch (trace(F^T F) - 3), term 1 the volume (det F - 1), each a compliant constraint with compliance
 // `relaxation` (the solver's soft_body_relaxation) scaled by the inverse rest volume.
-NB_D V3 tet_terms(const NbParticleDesc& pd, const float* xq, int i, int t, float dt, V3 delta) {
-    const int* ix = pd.tet_indices + 4 * t;
+NB_D void tet_term(const NbParticleDesc& pd, const float* xq, int i, int e, int term, float dt, ElemTerms& t) {
+    t.on = 0u;
+    const int* ix = pd.tet_indices + 4 * e;
     const V3 x0 = ld3(xq, ix[0]), x1 = ld3(xq, ix[1]), x2 = ld3(xq, ix[2]), x3 = ld3(xq, ix[3]);
     const float w[4] = {pd.particle_inv_mass[ix[0]], pd.particle_inv_mass[ix[1]], pd.particle_inv_mass[ix[2]],
                         pd.particle_inv_mass[ix[3]]};
     const M33 Ds = from_cols(sub(x1, x0), sub(x2, x0), sub(x3, x0));
     M33 Dm, inv_QT;
     for (int r = 0; r < 3; ++r)
-        for (int c = 0; c < 3; ++c) Dm.m[r][c] = pd.tet_poses[9 * t + 3 * r + c];
+        for (int c = 0; c < 3; ++c) Dm.m[r][c] = pd.tet_poses[9 * e + 3 * r + c];
     for (int r = 0; r < 3; ++r)
         for (int c = 0; c < 3; ++c) inv_QT.m[r][c] = Dm.m[c][r];
     const float inv_rest_volume = det3(Dm) * 6.0f;
     const M33 Fm = matmul3(Ds, Dm);
     const V3 f1 = col(Fm, 0), f2 = col(Fm, 1), f3 = col(Fm, 2);
     const float tr = dot(f1, f1) + dot(f2, f2) + dot(f3, f3);
-    for (int term = 0; term < 2; ++term) {
-        float C;
-        M33 dC;
-        if (term == 0) {
-            C = tr - 3.0f;
-            for (int r = 0; r < 3; ++r)
-                for (int c = 0; c < 3; ++c) dC.m[r][c] = Fm.m[r][c] * 2.0f;
-        } else {
-            C = det3(Fm) - 1.0f;
-            dC = from_cols(cross(f2, f3), cross(f3, f1), cross(f1, f2));
-        }
-        if (C == 0.0f) continue;
-        const M33 dP = matmul3(dC, inv_QT);
-        V3 grad[4];
-        grad[1] = col(dP, 0);
-        grad[2] = col(dP, 1);
-        grad[3] = col(dP, 2);
-        grad[0] = sub(sub(neg(grad[1]), grad[2]), grad[3]);
-        const float wsum = dot(grad[0], grad[0]) * w[0] + dot(grad[1], grad[1]) * w[1] +
-                           dot(grad[2], grad[2]) * w[2] + dot(grad[3], grad[3]) * w[3];
-        if (!(wsum > 0.0f)) continue;
-        float alpha = pd.soft_body_relaxation / dt / dt;
-        if (inv_rest_volume > 0.0f) alpha *= inv_rest_volume;
-        const float dlambda = -C / (wsum + alpha);
-        for (int r = 0; r < 4; ++r)
-            if (ix[r] == i) delta = add(delta, mul(grad[r], w[r] * dlambda));
+    float C;
+    M33 dC;
+    if (term == 0) {
+        C = tr - 3.0f;
+        for (int r = 0; r < 3; ++r)
+            for (int c = 0; c < 3; ++c) dC.m[r][c] = Fm.m[r][c] * 2.0f;
+    } else {
+        C = det3(Fm) - 1.0f;
+        dC = from_cols(cross(f2, f3), cross(f3, f1), cross(f1, f2));
     }
-    return delta;
+    if (C == 0.0f) return;
+    const M33 dP = matmul3(dC, inv_QT);
+    V3* grad = t.grad;
+    grad[1] = col(dP, 0);
+    grad[2] = col(dP, 1);
+    grad[3] = col(dP, 2);
+    grad[0] = sub(sub(neg(grad[1]), grad[2]), grad[3]);
+    const float wsum = dot(grad[0], grad[0]) * w[0] + dot(grad[1], grad[1]) * w[1] + dot(grad[2], grad[2]) * w[2] +
+                       dot(grad[3], grad[3]) * w[3];
+    if (!(wsum > 0.0f)) return;
+    float alpha = pd.soft_body_relaxation / dt / dt;
+    if (inv_rest_volume > 0.0f) alpha *= inv_rest_volume;
+    const float dlambda = -C / (wsum + alpha);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        t.mag[r] = w[r] * dlambda;
+        if (ix[r] == i) t.on |= 1u << r;
+    }
 }
 
-// Bending edges (bending_constraint, kernels.py:358-457), then tetrahedra, of one particle, added to its
-// delta after the constraint kernel's terms (the same order as one sequential sum); a kernel of its own
-// so that the constraint kernel keeps its register budget.  The solver zeroes the multipliers every iteration.
+// Bending edges, then tetrahedra, of one particle, added to its delta after the constraint kernel's terms
+// (the same order as one sequential sum): kElemGroup lanes per particle compute one element (one term of a
+// tetrahedron) each.  A kernel of its own so that the constraint kernel keeps its register budget.  The
+// solver zeroes the multipliers every iteration.
 __global__ void __launch_bounds__(kThreads) particle_bending_kernel(NbParticleDesc pd, NbParticleIO io, float dt) {
-    const int i = blockIdx.x * kThreads + threadIdx.x;
+    const int lane = threadIdx.x & (kElemGroup - 1);
+    const unsigned gmask = ((1u << kElemGroup) - 1u) << (threadIdx.x & 31 & ~(kElemGroup - 1));
+    const int i = blockIdx.x * kElemSlots + threadIdx.x / kElemGroup;
     if (i >= pd.particle_count) return;
     const int e_lo = pd.edge_count > 0 ? pd.particle_edge_start[i] : 0;
     const int e_hi = pd.edge_count > 0 ? pd.particle_edge_start[i + 1] : 0;
@@ -533,50 +798,26 @@ __global__ void __launch_bounds__(kThreads) particle_bending_kernel(NbParticleDe
     const float* xq = io.particle_q_out;
     const float* vq = io.particle_qd_out;
     V3 delta = ld3(io.delta, i);
-    {
-        for (int k = e_lo; k < e_hi; ++k) {
-            const int e = pd.particle_edge_list[k];
-            const int* ix = pd.edge_indices + 4 * e;
-            const float ke = pd.edge_bending_properties[2 * e], kd = pd.edge_bending_properties[2 * e + 1];
-            const V3 x1 = ld3(xq, ix[0]), x2 = ld3(xq, ix[1]), x3 = ld3(xq, ix[2]), x4 = ld3(xq, ix[3]);
-            const float w[4] = {pd.particle_inv_mass[ix[0]], pd.particle_inv_mass[ix[1]],
-                                pd.particle_inv_mass[ix[2]], pd.particle_inv_mass[ix[3]]};
-            const V3 n1 = cross(sub(x3, x1), sub(x4, x1));
-            const V3 n2 = cross(sub(x4, x2), sub(x3, x2));
-            const V3 ev = sub(x4, x3);
-            const float n1_length = length(n1), n2_length = length(n2), e_length = length(ev);
-            if (n1_length < 1.0e-6f || n2_length < 1.0e-6f || e_length < 1.0e-6f) continue;
-            const V3 n1_hat = divs(n1, n1_length), n2_hat = divs(n2, n2_length), e_hat = divs(ev, e_length);
-            const float cos_theta = dot(n1_hat, n2_hat);
-            const float sin_theta = dot(cross(n1_hat, n2_hat), e_hat);
-            const float c = nb_atan2(sin_theta, cos_theta) - pd.edge_rest_angle[e];
-            V3 grad[4];
-            grad[0] = mul(neg(n1_hat), e_length);
-            grad[1] = mul(neg(n2_hat), e_length);
-            grad[2] = sub(mul(neg(n1_hat), dot(sub(x1, x4), e_hat)), mul(n2_hat, dot(sub(x2, x4), e_hat)));
-            grad[3] = sub(mul(neg(n1_hat), dot(sub(x3, x1), e_hat)), mul(n2_hat, dot(sub(x3, x2), e_hat)));
-            const float denominator = w[0] * length_sq(grad[0]) + w[1] * length_sq(grad[1]) +
-                                      w[2] * length_sq(grad[2]) + w[3] * length_sq(grad[3]);
-            if (denominator <= 0.0f || ke <= 0.0f || kd < 0.0f) continue;
-            const float alpha = 1.0f / (ke * dt * dt);
-            const float gamma = kd / (ke * dt);
-            const float grad_dot_v = dt * (dot(grad[0], ld3(vq, ix[0])) + dot(grad[1], ld3(vq, ix[1])) +
-                                           dot(grad[2], ld3(vq, ix[2])) + dot(grad[3], ld3(vq, ix[3])));
-            const float lambda_prev = 0.0f;
-            const float dlambda =
-                -1.0f * (c + alpha * lambda_prev + gamma * grad_dot_v) / ((1.0f + gamma) * denominator + alpha);
-            for (int r = 0; r < 4; ++r)
-                if (ix[r] == i) delta = add(delta, mul(grad[r], w[r] * dlambda));
-        }
+    ElemTerms t;
+    for (int k = e_lo; k < e_hi; k += kElemGroup) {
+        t.on = 0u;
+        if (k + lane < e_hi) edge_terms(pd, xq, vq, i, pd.particle_edge_list[k + lane], dt, t);
+        delta = add_terms(t, gmask, min(e_hi - k, kElemGroup), delta);
     }
-    for (int k = t_lo; k < t_hi; ++k) delta = tet_terms(pd, xq, i, pd.particle_tet_list[k], dt, delta);
-    st3(io.delta, i, delta);
+    // two terms per tetrahedron: lane 2 a + term takes a term of the a-th
+    for (int k = 2 * t_lo; k < 2 * t_hi; k += kElemGroup) {
+        t.on = 0u;
+        if (k + lane < 2 * t_hi) tet_term(pd, xq, i, pd.particle_tet_list[(k + lane) >> 1], (k + lane) & 1, dt, t);
+        delta = add_terms(t, gmask, min(2 * t_hi - k, kElemGroup), delta);
+    }
+    if (lane == 0) st3(io.delta, i, delta);
 }
 
 // apply_particle_deltas (kernels.py:776-807), in place; then the particle enters the next cell table.
 __global__ void __launch_bounds__(kThreads) particle_apply_kernel(NbParticleDesc pd, NbParticleIO io, float dt,
                                                                   Grid g, int next_table, int insert) {
     const int p = blockIdx.x * kThreads + threadIdx.x;
+    if (p == 0 && g.sorted) g.cursor[0] = 0;  // for the next iteration's ranges
     if (p >= pd.particle_count || !active(pd, p)) return;
     const V3 x0 = ld3(io.particle_q, p);
     const V3 xp = ld3(io.particle_q_out, p);
@@ -644,6 +885,31 @@ bool check_pd(const NbParticleDesc* pd) {
     return true;
 }
 
+// Lays the neighbour search out in the caller's scratch: grid_head [2 n] and grid_next [P].  The sorted
+// form needs M <= P counts (grid_next) and M ranges + P entries (grid_head); M is the largest power of two
+// that fits, from a fourth of the particles up -- with fewer buckets its rows hold too many strangers,
+// and the lists, which use all n buckets, are taken (grid_size >= 2 P always fits).
+cudaError_t grid_layout(Grid& g, const NbParticleIO* io, int P, cudaStream_t st) {
+    const long long room = 2LL * io->grid_size - 2;  // ints, after the cursor and up to one to align
+    long long M = 1;
+    while (2 * M <= P) M *= 2;
+    while (M > 1 && 2 * M + 2LL * P > room) M /= 2;
+    g.sorted = M >= kMinSorted && 4 * M >= P && 2 * M + 2LL * P <= room;
+    if (!g.sorted) {
+        g.head = io->grid_head;
+        g.next = io->grid_next;
+        g.mask = (uint32_t)io->grid_size - 1u;
+        return cudaMemsetAsync(g.head, 0xff, sizeof(int32_t) * (size_t)io->grid_size, st);
+    }
+    int32_t* base = io->grid_head + (((uintptr_t)io->grid_head & 7u) ? 1 : 0);
+    g.range = reinterpret_cast<int2*>(base);
+    g.entry = g.range + M;
+    g.cursor = base + 2 * M + 2LL * P;
+    g.count = io->grid_next;
+    g.mask = (uint32_t)(M - 1);
+    return cudaMemsetAsync(g.count, 0, sizeof(int32_t) * (size_t)M, st);
+}
+
 }  // namespace
 
 extern "C" {
@@ -683,11 +949,8 @@ int nb_particle_step(const NbParticleDesc* pd, const NbParticleIO* io, const NbS
         const float h = 2.0f * pd->particle_max_radius + pd->particle_cohesion;
         const int32_t n = io->grid_size;
         if (!io->grid_head || !io->grid_next || n <= 0 || (n & (n - 1)) != 0 || !(h > 0.0f)) return NB_ERR_INVALID;
-        g.head = io->grid_head;
-        g.next = io->grid_next;
-        g.mask = (uint32_t)n - 1u;
         g.inv_h = 1.0f / h;
-        cudaError_t e = cudaMemsetAsync(g.head, 0xff, sizeof(int32_t) * (size_t)n, st);
+        const cudaError_t e = grid_layout(g, io, P, st);
         if (e != cudaSuccess) return nb_cuda_rc(e);
     }
     NbSoftContacts none{};
@@ -698,10 +961,17 @@ int nb_particle_step(const NbParticleDesc* pd, const NbParticleIO* io, const NbS
     const int con_blocks = (P + kSlots - 1) / kSlots;
     for (int it = 0; it < iterations; ++it) {
         const int table = it & 1;
-        particle_constraints_kernel<<<con_blocks, kThreads, 0, st>>>(*pd, *io, scv, has_sc, dt, relaxation, g,
-                                                                     table);
+        if (g.on && g.sorted) {
+            particle_ranges_kernel<<<(g.mask + kRangeBuckets) / kRangeBuckets, kThreads, 0, st>>>(g);
+            particle_scatter_kernel<<<blocks, kThreads, 0, st>>>(*pd, io->particle_q_out, g);
+            particle_constraints_kernel<true><<<con_blocks, kThreads, 0, st>>>(*pd, *io, scv, has_sc, dt, relaxation,
+                                                                               g, table);
+        } else {
+            particle_constraints_kernel<false><<<con_blocks, kThreads, 0, st>>>(*pd, *io, scv, has_sc, dt, relaxation,
+                                                                                g, table);
+        }
         if (pd->edge_count > 0 || pd->tet_count > 0)
-            particle_bending_kernel<<<blocks, kThreads, 0, st>>>(*pd, *io, dt);
+            particle_bending_kernel<<<(P + kElemSlots - 1) / kElemSlots, kThreads, 0, st>>>(*pd, *io, dt);
         particle_apply_kernel<<<blocks, kThreads, 0, st>>>(*pd, *io, dt, g, table ^ 1,
                                                            g.on && it + 1 < iterations ? 1 : 0);
     }
