@@ -30,14 +30,12 @@ namespace {
 
 constexpr int kST = NB_STEP_THREADS;  // threads per CTA
 
-// entries of one ordered batch per group: at least one test round of G items,
-// sized so that 8 warp groups' batches (21.5 KB) leave room for two CTAs' arenas per SM
 template <int G>
-struct BatchCap {
-    static constexpr int value = G == 32 ? 48 : (G == 256 ? 256 : 128);
-};
-template <int G>
-using Batch = nb::OrderedBatch<BatchCap<G>::value>;
+using Batch = nb::OrderedBatch<G>;
+
+// bit of the slab's body flags: the body's inertia and effective inverse inertia are finite (set when the
+// world is staged; apply_zero_delta asks for it every iteration)
+constexpr int kFiniteInertia = 1 << 30;
 
 // Per-world body state in shared memory.  kCompact = false: everything the
 // substep touches is staged (43 words per body); kCompact = true: only the
@@ -235,21 +233,15 @@ __device__ void apply_body_delta(TF& q, V3& v, V3& w, V3 dlin, V3 dang, float we
 // quaternion, the position re-expressed about the com, the velocities with +0 added and the rest
 // thresholds -- the inertia terms are skipped.  Otherwise the general form runs.
 __device__ void apply_zero_delta(TF& q, V3& v, V3& w, V3 com, const M33& I, float inv_m, const M33& inv_I,
-                                 float dt) {
+                                 bool finite_inertia, float dt) {
     if (inv_m == 0.0f) return;
     const Q4 q0 = q.q;
     const bool q_ok = q0.x != 0.0f && q0.y != 0.0f && q0.z != 0.0f && q0.w != 0.0f && isfinite(q0.x) &&
                       isfinite(q0.y) && isfinite(q0.z) && isfinite(q0.w);
     const bool w_ok = isfinite(w.x) && isfinite(w.y) && isfinite(w.z) && !(w.x == 0.0f && signbit(w.x)) &&
                       !(w.y == 0.0f && signbit(w.y)) && !(w.z == 0.0f && signbit(w.z));
-    // x * 0 is 0 for every finite x and NaN otherwise
-    float inert = 0.0f;
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) inert += I.m[r][c] * 0.0f + inv_I.m[r][c] * 0.0f;
     const V3 zero{0.0f, 0.0f, 0.0f};
-    if (!(q_ok && w_ok && inert == 0.0f)) {
+    if (!(q_ok && w_ok && finite_inertia)) {
         apply_body_delta(q, v, w, zero, zero, 1.0f, com, I, inv_m, inv_I, dt);
         return;
     }
@@ -264,6 +256,17 @@ __device__ void apply_zero_delta(TF& q, V3& v, V3& w, V3 com, const M33& I, floa
     if (length(w1) < 1e-4f) w1 = zero;
     v = v1;
     w = w1;
+}
+
+// whether a body's inertia and inverse inertia are finite
+__device__ __forceinline__ bool inertia_finite(const M33& I, const M33& inv_I) {
+    // x * 0 is 0 for every finite x and NaN otherwise
+    float inert = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) inert += I.m[r][c] * 0.0f + inv_I.m[r][c] * 0.0f;
+    return inert == 0.0f;
 }
 
 // kernels.py:1945-1979
@@ -369,7 +372,7 @@ __device__ void solve_contact(const NbModelDesc& m, const SB& S, float4 r0, floa
     float mu = 0.0f, mut = 0.0f, mur = 0.0f;
     if (sa >= 0) { nz += 1; mu += __ldg(m.shape_mu + sa); mut += __ldg(m.shape_mu_torsional + sa); mur += __ldg(m.shape_mu_rolling + sa); }
     if (sb >= 0) { nz += 1; mu += __ldg(m.shape_mu + sb); mut += __ldg(m.shape_mu_torsional + sb); mur += __ldg(m.shape_mu_rolling + sb); }
-    if (nz > 0) { mu /= (float)nz; mut /= (float)nz; mur /= (float)nz; }
+    if (nz == 2) { mu *= 0.5f; mut *= 0.5f; mur *= 0.5f; }  // the mean over the contact's shapes
     V3 r_a = sub(bx_a, tf_point(Xa, com_a));
     V3 r_b = sub(bx_b, tf_point(Xb, com_b));
     V3 ang_a = neg(cross(r_a, n));
@@ -1117,6 +1120,7 @@ __device__ __forceinline__ void step_world(const NbModelDesc& m, const NbXpbdPar
                 S.iI[k * nb + i] = kin ? 0.0f : m.body_inv_inertia[9 * (size_t)bi + k];
             }
         }
+        if (model_joints && inertia_finite(S.inertia(i), S.inv_inertia(i))) S.flags[i] = fl | kFiniteInertia;
         S.cnt[i] = 0;
     }
     const int j0 = m.world_joint_start[w], j1 = m.world_joint_start[w + 1];
@@ -1196,7 +1200,7 @@ __device__ __forceinline__ void step_world(const NbModelDesc& m, const NbXpbdPar
                 const float im = S.inv_m(i);
                 const M33 I = S.inertia(i), iI = S.inv_inertia(i);
                 apply_body_delta(q, v, wv, dl, da, weight, com, I, im, iI, dt);
-                if (model_joints && !world_joints) apply_zero_delta(q, v, wv, com, I, im, iI, dt);
+                if (model_joints && !world_joints) apply_zero_delta(q, v, wv, com, I, im, iI, (S.flags[i] & kFiniteInertia) != 0, dt);
                 S.set(i, q, v, wv);
             }
             group_sync<G>(g);

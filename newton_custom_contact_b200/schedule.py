@@ -31,9 +31,10 @@ SLAB_WORDS_PER_BODY = 6 + 13 + 4 + 9 + 9 + 1 + 1  # must match slab_words_per_bo
 SLAB_WORDS_COMPACT = 6 + 13 + 1 + 1  # slab_words_per_body<true>()
 STEP_MODES = {"batch": 0, "groups": 1, "groups_compact": 2}
 GROUP_MODE_SIZES = (32, 64, 128)
-# The step kernel's static shared memory (the groups' ordered-accumulation batches) is 21.8 KB for
-# 32-thread groups and up to 28.9 KB for 64-thread groups; with the dynamic arena below, two CTAs
-# still fit one SM's 228 KB.
+# The step kernel's static shared memory (the groups' ordered-accumulation rings) is 19 KB for 32-thread
+# groups, 21 KB for 64, 25 KB for 128 and 33 KB for 256; with the dynamic arena below, two CTAs of up to
+# 128-thread groups still fit one SM's 228 KB (a 256-thread group's CTA holds one world and takes only
+# that world's room).
 ARENA_WORDS_TWO_CTAS = 21 * 1024  # 84 KB: two CTAs per SM
 ARENA_WORDS_MAX = 48 * 1024       # 192 KB: the opt-in per-CTA maximum less the kernel's static shared memory
 GROUP_SIZES = (32, 64, 128, 256)
@@ -84,10 +85,39 @@ def group_share_words(group_threads: int, arena_words: int = ARENA_WORDS_TWO_CTA
     return (arena_words // (CTA_THREADS // group_threads)) & ~1
 
 
-def default_mode(max_world_bodies: int) -> tuple:
-    """(mode, group_threads): the smallest group whose share holds the largest world, with the full
-    slab if it fits, else the compact one; else batches.  (Measured on the 4096-world drop: one
-    warp per world with the compact slab beats 64-thread groups with the full slab.)"""
+def default_mode(max_world_bodies: int, world_count: int, sms: int | None = None) -> tuple:
+    """(mode, group_threads) of the step for `world_count` worlds of at most `max_world_bodies` bodies.
+
+    The kernel is bound by each world's chain of dependent instructions, which a wider group shortens,
+    until the worlds no longer run all at once (2 CTAs of 256 threads per SM, so 2, 4, 8, 16 groups of
+    256, 128, 64, 32 threads): the widest group that runs every world at once is taken.  Worlds of more
+    than 64 bodies keep 64 threads for as long as one warp per world would not need a second round
+    either (their body passes take three warp rounds or more); smaller ones change over at once.
+    Measured (148 SMs, 8 iterations, us per step at 256 / 128 / 64 / 32 threads; mixed shapes, 8..128 and
+    8..32 bodies):
+
+        worlds   8..128 bodies            8..32 bodies
+        37        59 /  70 /  94 / 135     57 /  61 /  65 /  69
+        150       64 /  79 / 104 / 159     57 /  62 /  66 /  72
+        600      146 /  97 / 118 / 189    130 /  88 /  78 /  84
+        1024     213 / 138 / 119 / 191    192 / 115 /  79 /  89
+        1600     318 / 205 / 155 / 203    285 / 170 / 111 /  95
+        4096     817 / 521 / 361 / 304    682 / 410 / 240 / 159
+
+    Within the group modes the full slab is taken where it fits a group's share, else the compact one
+    (they differ by a few percent); 256 threads and worlds beyond every share run as batches."""
+    sms = sms or _sm_count()
+    if world_count <= 2 * sms:
+        return "batch", 256
+    for g in (128, 64, 32):
+        slots = sms * 2 * (CTA_THREADS // g)
+        if g == 64 and max_world_bodies > 64:
+            slots *= 2
+        if world_count <= slots or g == 32:
+            for words, mode in ((SLAB_WORDS_PER_BODY, "groups"), (SLAB_WORDS_COMPACT, "groups_compact")):
+                if words * max_world_bodies <= group_share_words(g):
+                    return mode, g
+    # more worlds than fit at once, too large for one warp's share: the smallest group that holds them
     for g in GROUP_MODE_SIZES:
         for words, mode in ((SLAB_WORDS_PER_BODY, "groups"), (SLAB_WORDS_COMPACT, "groups_compact")):
             if words * max_world_bodies <= group_share_words(g):
@@ -104,7 +134,7 @@ def build_schedule(model, group_threads: int | None = None, mode: str | None = N
         if group_threads is not None:
             mode = "batch"
         else:
-            mode, group_threads = default_mode(maxb)
+            mode, group_threads = default_mode(maxb, W)
     if mode not in STEP_MODES:
         raise ValueError(f"mode must be one of {tuple(STEP_MODES)}")
     if mode != "batch":
@@ -125,7 +155,8 @@ def build_schedule(model, group_threads: int | None = None, mode: str | None = N
     slab = SLAB_WORDS_PER_BODY * np.maximum(nb, 1)
     slab = slab + (slab & 1)  # keep every slab 8-byte aligned (int64 accumulators first)
     big = int(slab.max()) if W else 2
-    arena = ARENA_WORDS_TWO_CTAS if big <= ARENA_WORDS_TWO_CTAS else big
+    # a CTA that holds one world needs room for the largest one only
+    arena = big if groups == 1 or big > ARENA_WORDS_TWO_CTAS else ARENA_WORDS_TWO_CTAS
     if arena > ARENA_WORDS_MAX:
         raise ValueError(f"a world with {int(nb.max())} bodies does not fit in one CTA's shared memory")
     order = np.argsort(-nb, kind="stable")
