@@ -656,11 +656,14 @@ __device__ void vjp_integrate(const float* s, const float* f, V3 com, const M33&
     (void)x0;
 }
 
-// contact: inputs A pose (7) + A omega (3) + B pose (7) + B omega (3); outputs the four deltas (12)
+// contact: inputs A pose (7) + A omega (3) + B pose (7) + B omega (3); outputs the four deltas (12).
+// The inputs j0 .. j0 + kDirs - 1 (a chunk) of the 20: kChunks chunks make the whole.
+constexpr int kChunks = (20 + kDirs - 1) / kDirs;
+
+template <int j0>
 __device__ __forceinline__ void vjp_contact(const ContactC& c, const float* sa, const float* sb, float relaxation, float dt,
                             const float* gout, float* ga, float* gb) {
-#pragma unroll
-    for (int j0 = 0; j0 < 20; j0 += kDirs) {
+    {
         BodyT<Dual<kDirs>> A, B;
         A.p = {seed<kDirs>(sa[0], 0, j0), seed<kDirs>(sa[1], 1, j0), seed<kDirs>(sa[2], 2, j0)};
         A.r = {seed<kDirs>(sa[3], 3, j0), seed<kDirs>(sa[4], 4, j0), seed<kDirs>(sa[5], 5, j0),
@@ -987,9 +990,11 @@ __global__ void __launch_bounds__(kThreads) adjoint_bodies_kernel(NbModelDesc m,
     }
 }
 
-// active contacts of iteration it: VJP of the contact's deltas into its bodies' poses and angular velocities
-__global__ void __launch_bounds__(kThreads) adjoint_contacts_kernel(NbModelDesc m, NbXpbdParams p, NbAdjointIO io,
-                                                                    NbContactSeg seg, int it, float dt) {
+// active contacts of iteration it: VJP of the contact's deltas into its bodies' poses and angular
+// velocities, the inputs of one chunk
+template <int kChunk>
+__device__ __forceinline__ void adjoint_contacts(const NbModelDesc& m, const NbXpbdParams& p, const NbAdjointIO& io,
+                                                 const NbContactSeg& seg, int it, float dt) {
     const size_t B = (size_t)m.body_count;
     const float* S_it = io.tape_state + (size_t)it * B * 13;
     int n = io.active_count[it];
@@ -1011,8 +1016,8 @@ __global__ void __launch_bounds__(kThreads) adjoint_contacts_kernel(NbModelDesc 
             gout[6 + q] = dyn_b ? io.tape_delta[((size_t)it * B + b0 + c.lb) * 6 + q] : 0.0f;
         }
         float ga[13] = {}, gb[13] = {};
-        vjp_contact(c, sa, sb, p.rigid_contact_relaxation, dt, gout, ga, gb);
-        if (io.grad_shape_mu && c.mu > 0.0f) {
+        vjp_contact<kChunk * kDirs>(c, sa, sb, p.rigid_contact_relaxation, dt, gout, ga, gb);
+        if (kChunk == 0 && io.grad_shape_mu && c.mu > 0.0f) {
             // the contact's mu is the mean of its shapes' (kernels.py:2160-2178)
             const float gmu = vjp_contact_mu(c, sa, sb, p.rigid_contact_relaxation, dt, gout);
             if (gmu != 0.0f) {
@@ -1028,6 +1033,21 @@ __global__ void __launch_bounds__(kThreads) adjoint_contacts_kernel(NbModelDesc 
         if (dyn_b)
             for (int q = 0; q < 13; ++q)
                 if (gb[q] != 0.0f) atomicAdd(io.grad_acc + 13 * (size_t)(b0 + c.lb) + q, (double)gb[q]);
+    }
+}
+
+// One block row per chunk: a contact's chunks, each a pass over the whole contact with dual numbers, run
+// on kChunks threads at once instead of one after another.  Bound by that chain: with some 20,000 active
+// contacts one thread per contact is one warp per scheduler (256 stacks of 16 boxes: 46 us per launch).
+__global__ void __launch_bounds__(kThreads) adjoint_contacts_kernel(NbModelDesc m, NbXpbdParams p, NbAdjointIO io,
+                                                                    NbContactSeg seg, int it, float dt) {
+    static_assert(kChunks == 5, "one case per chunk");
+    switch (blockIdx.y) {
+        case 0: return adjoint_contacts<0>(m, p, io, seg, it, dt);
+        case 1: return adjoint_contacts<1>(m, p, io, seg, it, dt);
+        case 2: return adjoint_contacts<2>(m, p, io, seg, it, dt);
+        case 3: return adjoint_contacts<3>(m, p, io, seg, it, dt);
+        case 4: return adjoint_contacts<4>(m, p, io, seg, it, dt);
     }
 }
 
@@ -1074,7 +1094,7 @@ cudaError_t nb_launch_xpbd_adjoint(const NbModelDesc* m, const NbXpbdParams* p, 
     for (int it = K - 1; it >= 0; --it) {
         adjoint_bodies_kernel<<<gb, kThreads, 0, s>>>(*m, *io, it, has_contacts, dt);
         if (has_contacts && io->active_capacity > 0)
-            adjoint_contacts_kernel<<<gc, kThreads, 0, s>>>(*m, *p, *io, *seg, it, dt);
+            adjoint_contacts_kernel<<<dim3(gc, kChunks), kThreads, 0, s>>>(*m, *p, *io, *seg, it, dt);
     }
     adjoint_integrate_kernel<<<gb, kThreads, 0, s>>>(*m, *p, *io, dt);
     return cudaGetLastError();
