@@ -1038,7 +1038,8 @@ __device__ __forceinline__ void adjoint_contacts(const NbModelDesc& m, const NbX
 
 // One block row per chunk: a contact's chunks, each a pass over the whole contact with dual numbers, run
 // on kChunks threads at once instead of one after another.  Bound by that chain: with some 20,000 active
-// contacts one thread per contact is one warp per scheduler (256 stacks of 16 boxes: 46 us per launch).
+// contacts one thread per contact is one warp per scheduler (256 stacks of 16 boxes: 46 us per launch; in chunks of four
+// directions 31, of two 40).
 __global__ void __launch_bounds__(kThreads) adjoint_contacts_kernel(NbModelDesc m, NbXpbdParams p, NbAdjointIO io,
                                                                     NbContactSeg seg, int it, float dt) {
     static_assert(kChunks == 5, "one case per chunk");

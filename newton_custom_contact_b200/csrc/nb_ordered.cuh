@@ -115,6 +115,11 @@ __device__ __forceinline__ void ordered_flush(OrderedBatch<G>& B, int head, int 
         if (la >= 0) atomicOr(&B.own_a[t >> 5][la & (G - 1)], bit);
         if (lb >= 0) atomicOr(&B.own_b[t >> 5][lb & (G - 1)], bit);
     }
+    // Never taken (m > 0).  With a single call site the compiler merges the solve's products with the
+    // code around it and contracts other pairs of them into FMAs than in the other kernels that call it;
+    // a second site keeps one form, so that the product build's results are the same bits for every group
+    // size and from build to build.
+    if (m < 0) solve(t, B.d[t]);
     ordered_sync<G, kCTA>(g);  // the rows and the marks are visible
 #pragma unroll
     for (int w = 0; w < kW; ++w) {
@@ -138,22 +143,20 @@ __device__ __forceinline__ void ordered_flush(OrderedBatch<G>& B, int head, int 
 template <int G, int kCTA, class Test, class Solve, class Add>
 __device__ __forceinline__ void ordered_pass(OrderedBatch<G>& B, int n_items, int g, int t, Test& test, Solve& solve,
                                              Add& add) {
-    // the two flushes keep the solve out of line, which fixes how the product build contracts its sums
-    // (one flush in a loop of its own inlines it and moves results in the last bits)
     int n = 0, head = 0, round = 0;
-    for (int base = 0; base < n_items; base += G) {
-        if (n >= G) {
-            ordered_flush<G, kCTA>(B, head, G, g, t, solve, add);
-            head += G;
-            n -= G;
+    int base = 0;
+    // one flush for full rounds and the last, partial one: the solve is the step's longest code, and two
+    // live copies of it cost instruction fetches (4096 mixed worlds: 396 against 355 us per step)
+    for (;;) {
+        while (n < G && base < n_items) {
+            const int k = base + t;
+            int ends = 0;
+            const bool active = k < n_items && test(k, ends);
+            ordered_append<G, kCTA>(B, active, k, ends, g, t, head, round, n);
+            base += G;
+            ++round;
         }
-        const int k = base + t;
-        int ends = 0;
-        const bool active = k < n_items && test(k, ends);
-        ordered_append<G, kCTA>(B, active, k, ends, g, t, head, round, n);
-        ++round;
-    }
-    while (n > 0) {
+        if (n == 0) break;
         const int m = n < G ? n : G;
         ordered_flush<G, kCTA>(B, head, m, g, t, solve, add);
         head += m;
