@@ -244,8 +244,10 @@ __device__ void world_by_warp(const NbModelDesc& m, const float* __restrict__ bo
 
 // one large world by the whole CTA: shapes staged once, the pair chunks split
 // into one contiguous run per warp; pass 1 counts each run's hits, a scan over
-// the warps gives every run its first candidate index, pass 2 re-tests (a few
-// comparisons per pair) and writes -- the candidates stay in pair order
+// the warps gives every run its first candidate index, pass 2 writes -- the
+// candidates stay in pair order.  Pass 2 takes the hits from registers for the
+// first 8 chunks of a run (worlds of up to 8192 pairs, 128 bodies); what a
+// larger world has beyond is tested again
 __device__ void world_by_cta(const NbModelDesc& m, const float* __restrict__ body_q, const NbContactSeg& seg, int k,
                              float4* lo, float4* hi, QueueStage& st, int* s_run, int warp, int lane) {
     const unsigned* pairs = m.pair_shapes;
@@ -261,6 +263,9 @@ __device__ void world_by_cta(const NbModelDesc& m, const float* __restrict__ bod
     constexpr int kWarps = kBT / 32;
     const int per = (nchunks + kWarps - 1) / kWarps;
     const int c0 = warp * per, c1 = min(nchunks, c0 + per);
+    // the first kKept chunks' hit and easy bits (4 + 4 a chunk) stay in registers for pass 2
+    constexpr int kKept = 8;
+    unsigned kept[kKept / 4] = {};
     int count = 0;
     for (int c = c0; c < c1; ++c) {
         const int q = cbase + 128 * c + lane;
@@ -270,6 +275,9 @@ __device__ void world_by_cta(const NbModelDesc& m, const float* __restrict__ bod
         unsigned hit, easy;
         test_pairs(pw, q, p1, lo, hi, ns, seg.status, hit, easy);
         count += __popc(hit);
+        const unsigned bits = (hit | (easy << 4)) << (8 * ((c - c0) & 3));
+        if (c - c0 < 4) kept[0] |= bits;
+        else if (c - c0 < 8) kept[1] |= bits;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(kFull, count, o);
@@ -285,11 +293,17 @@ __device__ void world_by_cta(const NbModelDesc& m, const float* __restrict__ bod
     int ncand = 0;
     for (int c = c0; c < c1; ++c) {
         const int q = cbase + 128 * c + lane;
-        unsigned pw[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) pw[r] = q + 32 * r < p1 ? pairs[q + 32 * r] : 0u;
         unsigned hit, easy;
-        test_pairs(pw, q, p1, lo, hi, ns, seg.status, hit, easy);
+        if (c - c0 < kKept) {
+            const unsigned bits = (c - c0 < 4 ? kept[0] : kept[1]) >> (8 * ((c - c0) & 3));
+            hit = bits & 15u;
+            easy = (bits >> 4) & 15u;
+        } else {
+            unsigned pw[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) pw[r] = q + 32 * r < p1 ? pairs[q + 32 * r] : 0u;
+            test_pairs(pw, q, p1, lo, hi, ns, seg.status, hit, easy);
+        }
         int tot_h;
         emit_chunk(seg, queue, gjk_back, st, q, hit, easy, w, p0 + first + ncand, lane, tot_h);
         ncand += tot_h;
@@ -889,79 +903,96 @@ __global__ void __launch_bounds__(1024) world_scan_kernel(int W, int32_t* __rest
 }
 
 // Dense public Contacts arrays ordered by (world, key), and the same contacts
-// as solver records (rec), contiguous per world; one warp per world.  The
-// warp scans the contact counts of 32 candidates at a time, then its lanes
-// take the chunk's outputs in order (lane k writes output k, k + 32, ...),
-// each finding its candidate among the 32 scanned counts, so consecutive
-// lanes store to consecutive rows of every array.
-__global__ void __launch_bounds__(256) publish_kernel(NbModelDesc m, NbContactSeg seg, NbContactsPublic pub) {
-    const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
+// as solver records (rec), contiguous per world; one CTA per world.  Each warp
+// scans the contact counts of 32 candidates, the warps' totals give every warp
+// its first output, then a warp's lanes take its outputs in order (lane k
+// writes output k, k + 32, ...), each finding its candidate by a binary search
+// of the scanned counts, so consecutive lanes store to consecutive rows of
+// every array.  Bound by the latency of the counts' and slots' loads, one round
+// after another: 1 / 2 / 4 / 8 warps per world take 71 / 65 / 57 / 56 us for
+// 4096 worlds (180 MB), 11 / - / - / 4 us for one.
+constexpr int kPubT = 256;
+
+__global__ void __launch_bounds__(kPubT) publish_kernel(NbModelDesc m, NbContactSeg seg, NbContactsPublic pub) {
+    constexpr int kWarps = kPubT / 32;
+    __shared__ int s_tot[2][kWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int w = blockIdx.x;
+    if (w >= m.world_count) return;
     const float4* slots = reinterpret_cast<const float4*>(seg.slots);
     float4* rec = reinterpret_cast<float4*>(seg.rec);
-    for (int w = gw; w < m.world_count; w += nw) {
-        const int c0 = m.world_pair_start[w];
-        // a world's candidates never exceed its pairs, a candidate's contacts never exceed 5; the
-        // clamps keep corrupted counts from indexing past the slots
-        const int npair = m.world_pair_start[w + 1] - c0;
-        int nc = seg.cand_count[w];
-        nc = nc < 0 ? 0 : (nc > npair ? npair : nc);
-        const int64_t dst0 = pub.world_offset[w];
-        int64_t running = 0;
-        for (int base = 0; base < nc; base += 32) {
-            const int i = base + lane;
-            int n = i < nc ? (int)seg.counts[c0 + i] : 0;
-            n = n > 5 ? 5 : n;
-            int x = n;  // inclusive scan of the chunk's counts
+    const int c0 = m.world_pair_start[w];
+    // a world's candidates never exceed its pairs, a candidate's contacts never exceed 5; the
+    // clamps keep corrupted counts from indexing past the slots
+    const int npair = m.world_pair_start[w + 1] - c0;
+    int nc = seg.cand_count[w];
+    nc = nc < 0 ? 0 : (nc > npair ? npair : nc);
+    const int64_t dst0 = pub.world_offset[w];
+    int64_t running = 0;
+    int round = 0;
+    for (int base = 0; base < nc; base += 32 * kWarps) {
+        const int first = base + 32 * warp;
+        const int i = first + lane;
+        int n = i < nc ? (int)seg.counts[c0 + i] : 0;
+        n = n > 5 ? 5 : n;
+        int x = n;  // inclusive scan of the warp's counts
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int y = __shfl_up_sync(kFull, x, o);
-                if (lane >= o) x += y;
-            }
-            const int tot = __shfl_sync(kFull, x, 31);
-            for (int o0 = 0; o0 < tot; o0 += 32) {
-                const int o = o0 + lane;
-                // source lane: the number of lanes whose inclusive sum is <= o
-                int src = 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            int y = __shfl_up_sync(kFull, x, o);
+            if (lane >= o) x += y;
+        }
+        const int tot = __shfl_sync(kFull, x, 31);
+        int64_t at = dst0 + running;
+        // the totals of two rounds alternate, so one barrier per round is enough
+        if (lane == 0) s_tot[round & 1][warp] = tot;
+        __syncthreads();
 #pragma unroll
-                for (int k = 0; k < 32; ++k) src += __shfl_sync(kFull, x, k) <= o ? 1 : 0;
-                const int src_c = src < 31 ? src : 31;
-                const int x_src = __shfl_sync(kFull, x, src_c);
-                const int n_src = __shfl_sync(kFull, n, src_c);
-                if (o >= tot) continue;
-                const int j = o - (x_src - n_src);
-                const int64_t d = dst0 + running + o;
-                const float4* sl = slots + ((size_t)(c0 + base + src) * 5 + j) * 5;
-                const float4 a = sl[0], b = sl[1], c = sl[2], e = sl[3], f = sl[4];
-                // solver record: the tag moves next to the normal so the
-                // penetration test reads the first 48 bytes only
-                // rec and the public rows hold the first `capacity` contacts (world_scan_kernel flagged
-                // an overflow and clamped the worlds' solver counts; a negative offset is corrupt)
-                if (d < 0 || d >= pub.capacity) continue;
-                float4* r = rec + (size_t)d * 5;
-                r[0] = a;
-                r[1] = b;
-                r[2] = make_float4(c.x, c.y, c.z, f.w);
-                r[3] = make_float4(e.x, e.y, e.z, c.w);
-                r[4] = make_float4(f.x, f.y, f.z, e.w);
-                if (seg.rec_index) seg.rec_index[d] = (int32_t)d;
-                const int s0 = __float_as_int(c.w), s1 = __float_as_int(e.w);
-                pub.shape0[d] = s0;
-                pub.shape1[d] = s1;
-                pub.point0[3 * d] = a.x; pub.point0[3 * d + 1] = a.y; pub.point0[3 * d + 2] = a.z;
-                pub.point1[3 * d] = b.x; pub.point1[3 * d + 1] = b.y; pub.point1[3 * d + 2] = b.z;
-                pub.normal[3 * d] = c.x; pub.normal[3 * d + 1] = c.y; pub.normal[3 * d + 2] = c.z;
-                pub.offset0[3 * d] = e.x; pub.offset0[3 * d + 1] = e.y; pub.offset0[3 * d + 2] = e.z;
-                pub.offset1[3 * d] = f.x; pub.offset1[3 * d + 1] = f.y; pub.offset1[3 * d + 2] = f.z;
-                pub.margin0[d] = a.w;
-                pub.margin1[d] = b.w;
-                if (pub.sort_key) {
-                    const int sub = (__float_as_int(f.w) >> 24) & 0xFF;
-                    pub.sort_key[d] = ((int64_t)(s0 & 0xFFFFF) << 43) | ((int64_t)(s1 & 0xFFFFF) << 23) | (int64_t)sub;
-                }
+        for (int k = 0; k < kWarps; ++k) {
+            const int v = s_tot[round & 1][k];
+            if (k < warp) at += v;
+            running += v;
+        }
+        ++round;
+        for (int o0 = 0; o0 < tot; o0 += 32) {
+            const int o = o0 + lane;
+            // source lane: the number of lanes whose inclusive sum is <= o
+            int src = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(kFull, x, src + step - 1) <= o) src += step;
+            const int x_src = __shfl_sync(kFull, x, src);
+            const int n_src = __shfl_sync(kFull, n, src);
+            if (o >= tot) continue;
+            const int j = o - (x_src - n_src);
+            const int64_t d = at + o;
+            const float4* sl = slots + ((size_t)(c0 + first + src) * 5 + j) * 5;
+            const float4 a = sl[0], b = sl[1], c = sl[2], e = sl[3], f = sl[4];
+            // solver record: the tag moves next to the normal so the
+            // penetration test reads the first 48 bytes only
+            // rec and the public rows hold the first `capacity` contacts (world_scan_kernel flagged
+            // an overflow and clamped the worlds' solver counts; a negative offset is corrupt)
+            if (d < 0 || d >= pub.capacity) continue;
+            float4* r = rec + (size_t)d * 5;
+            r[0] = a;
+            r[1] = b;
+            r[2] = make_float4(c.x, c.y, c.z, f.w);
+            r[3] = make_float4(e.x, e.y, e.z, c.w);
+            r[4] = make_float4(f.x, f.y, f.z, e.w);
+            if (seg.rec_index) seg.rec_index[d] = (int32_t)d;
+            const int s0 = __float_as_int(c.w), s1 = __float_as_int(e.w);
+            pub.shape0[d] = s0;
+            pub.shape1[d] = s1;
+            pub.point0[3 * d] = a.x; pub.point0[3 * d + 1] = a.y; pub.point0[3 * d + 2] = a.z;
+            pub.point1[3 * d] = b.x; pub.point1[3 * d + 1] = b.y; pub.point1[3 * d + 2] = b.z;
+            pub.normal[3 * d] = c.x; pub.normal[3 * d + 1] = c.y; pub.normal[3 * d + 2] = c.z;
+            pub.offset0[3 * d] = e.x; pub.offset0[3 * d + 1] = e.y; pub.offset0[3 * d + 2] = e.z;
+            pub.offset1[3 * d] = f.x; pub.offset1[3 * d + 1] = f.y; pub.offset1[3 * d + 2] = f.z;
+            pub.margin0[d] = a.w;
+            pub.margin1[d] = b.w;
+            if (pub.sort_key) {
+                const int sb = (__float_as_int(f.w) >> 24) & 0xFF;
+                pub.sort_key[d] = ((int64_t)(s0 & 0xFFFFF) << 43) | ((int64_t)(s1 & 0xFFFFF) << 23) | (int64_t)sb;
             }
-            running += tot;
         }
     }
 }
@@ -1155,9 +1186,8 @@ cudaError_t nb_launch_collide(const NbModelDesc* m, const float* body_q, const N
     NarrowOccupancy occ;
     e = narrow_occupancy(&occ);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(seg->work_counter, 0, 4 * sizeof(int32_t), stream);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(seg->work_counter + 5, 0, 3 * sizeof(int32_t), stream);
+    // one memset for all counters ([4] is the step's, which clears it itself)
+    e = cudaMemsetAsync(seg->work_counter, 0, 8 * sizeof(int32_t), stream);
     if (e != cudaSuccess) return e;
     const int sms = sm_count();
     if (sap) broadphase_kernel<true><<<sms * 4, kBT, smem, stream>>>(*m, body_q, *seg);
@@ -1183,8 +1213,8 @@ cudaError_t nb_launch_publish(const NbModelDesc* m, const NbContactSeg* seg, con
                                               pub->count, pub->capacity, seg->status, pub->generation);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const int blocks = (m->world_count * 32 + 255) / 256;
-    publish_kernel<<<blocks < 1 ? 1 : blocks, 256, 0, stream>>>(*m, *seg, *pub);
+    const int worlds = m->world_count < 1 ? 1 : m->world_count;
+    publish_kernel<<<worlds, kPubT, 0, stream>>>(*m, *seg, *pub);
     return cudaGetLastError();
 }
 
