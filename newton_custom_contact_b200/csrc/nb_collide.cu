@@ -39,8 +39,11 @@ using namespace nbg;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kBT = 256;             // broad phase: threads per CTA (8 worlds in flight)
 constexpr int kNT = 128;             // narrow phase: threads per CTA
-constexpr int kGjkMinBlocks = 12;     // MPR/GJK kernel: resident CTAs per SM the registers are fitted to
-constexpr int kManifoldMinBlocks = 5;   // manifold kernel (96 registers: fewer, heavier threads measure faster)
+// MPR/GJK and manifold kernels: resident CTAs per SM the registers are fitted to, for few and for many
+// bodies (narrow_is_small below)
+constexpr int kAnalyticBlocks = 8;  // 64 registers: 4096 worlds 510 us per collide, 520 at 5 or 10 CTAs per SM
+constexpr int kGjkBlocksFew = 4, kGjkBlocksMany = 8;
+constexpr int kManifoldBlocksFew = 2, kManifoldBlocksMany = 4;
 constexpr int kSlotF4 = 25;          // 5 contacts x 5 float4 per candidate
 
 __device__ __forceinline__ void store_geom(float4* g, const Geom& x) {
@@ -626,7 +629,7 @@ __device__ __forceinline__ void narrow_finish(const NbContactSeg& seg, const Nar
 
 // analytic queue: sphere / capsule / plane pairs; a plane-box pair with no
 // corner inside the gap is forwarded to the MPR/GJK queue (narrow_phase.py:598-603)
-__global__ void __launch_bounds__(kNT)
+__global__ void __launch_bounds__(kNT, kAnalyticBlocks)
 narrow_analytic_kernel(NbModelDesc m, const float* __restrict__ body_q, NbContactSeg seg) {
     const int n0 = seg.work_counter[2];
     const int P = m.pair_count;
@@ -778,52 +781,109 @@ gjk_prefilter_kernel(NbModelDesc m, NbContactSeg seg) {
 // queue's back half, which the prefilter has consumed: box-box items from
 // the top down, the others from the bottom of that region up (the items
 // never exceed the n1 <= pair_count entries the region held).
-// Latency and divergence bound: 12 CTAs per SM (48 warps, 40 registers, a
-// few bytes of spills) hide more of it than 6, 8, 10 or 16 (measured) or the
-// unconstrained 122 registers at 4 CTAs.
-__global__ void __launch_bounds__(kNT, kGjkMinBlocks)
+// Latency and divergence bound: with more items than threads, resident warps
+// hide it (64 registers, 8 CTAs per SM); with fewer, each item's own chain is
+// the kernel's time, and registers without spills shorten it (128, 4 CTAs).
+// The few-bodies variant also shares an item between two warps while there are
+// threads for that: one runs MPR, the other GJK at the same time (MPR finds no
+// overlap in 97 % or more of the items, so GJK's result is almost always used):
+// one world of 64 boxes 30 -> 22 us, 256 stacks of 16 boxes 32 -> 20 us.  With
+// more items than that the shared items only cost barriers and registers (300
+// worlds of 64 boxes 335 -> 352 us for two collides, 4096 mixed ones 510 -> 549).
+
+// what becomes of an item after MPR / GJK: its single contact, or its place in the manifold queue
+__device__ __forceinline__ void gjk_hand_off(const NbContactSeg& seg, NarrowItem& it, bool live, bool ready,
+                                             const GjkSetup& s, V3 pa, V3 pb, V3 nrm, float sd, bool box, int2 e,
+                                             int2* queue, long long top, int n1, int lane) {
+    const bool manifold = ready && gjk_finish(it.wr, s, pa, pb, nrm, sd);
+    if (manifold) {
+        float4* h = it.wr.slots + kSlotF4 - 3;
+        h[0] = make_float4(pa.x, pa.y, pa.z, 0.0f);
+        h[1] = make_float4(pb.x, pb.y, pb.z, 0.0f);
+        h[2] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
+    } else if (live) {
+        narrow_finish(seg, it);
+    }
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned bb = __ballot_sync(kFull, manifold && box);
+    const unsigned bo = __ballot_sync(kFull, manifold && !box);
+    int ob = 0, oo = 0;
+    if (lane == 0 && bb) ob = atomicAdd(&seg.work_counter[1], __popc(bb));
+    if (lane == 0 && bo) oo = atomicAdd(&seg.work_counter[7], __popc(bo));
+    ob = __shfl_sync(kFull, ob, 0);
+    oo = __shfl_sync(kFull, oo, 0);
+    if (manifold && box) queue[top - (ob + __popc(bb & below))] = e;
+    if (manifold && !box) queue[top - n1 + 1 + (oo + __popc(bo & below))] = e;
+}
+
+template <int kMinBlocks>
+__global__ void __launch_bounds__(kNT, kMinBlocks)
 narrow_gjk_kernel(NbModelDesc m, const float* __restrict__ body_q, NbContactSeg seg) {
     const int n_box = seg.work_counter[5], n_other = seg.work_counter[6], n1 = seg.work_counter[3];
     const int n = n_box + n_other;
     int2* queue = reinterpret_cast<int2*>(seg.queue);
     const long long top = 2 * (long long)m.pair_count - 1;
     const int lane = threadIdx.x & 31;
+    if constexpr (kMinBlocks == kGjkBlocksFew) {
+        constexpr int kItems = kNT / 2;
+        __shared__ float s_gjk[10][kItems];  // GJK's witness points, normal and distance
+        if (n <= (int)gridDim.x * kItems) {
+            const int slot = threadIdx.x % kItems;
+            const bool first = threadIdx.x < kItems;  // MPR and the rest of the item; the other half: GJK
+            const int i = blockIdx.x * kItems + slot;
+            const bool box = i < n_box;
+            int2 e = make_int2(0, 0);
+            NarrowItem it;
+            GjkSetup s;
+            bool live = false, ready = false, overlap = false;
+            V3 pa{0, 0, 0}, pb{0, 0, 0}, nrm{0, 0, 0};
+            float sd = 0.0f;
+            if (i < n) {
+                e = box ? queue[i] : queue[n1 - 1 - (i - n_box)];
+                live = narrow_setup(m, seg, body_q, e, it);
+                ready = live && gjk_prepare(it.ga, it.gb, s);
+            }
+            if (ready && first) overlap = mpr_stage(s, pa, pb, nrm, sd);
+            if (ready && !first) {
+                gjk_core(s.p, 0.0f, pa, pb, nrm, sd);
+                const float v[10] = {pa.x, pa.y, pa.z, pb.x, pb.y, pb.z, nrm.x, nrm.y, nrm.z, sd};
+#pragma unroll
+                for (int k = 0; k < 10; ++k) s_gjk[k][slot] = v[k];
+            }
+            __syncthreads();
+            if (!first) return;
+            if (ready && !overlap) {
+                pa = V3{s_gjk[0][slot], s_gjk[1][slot], s_gjk[2][slot]};
+                pb = V3{s_gjk[3][slot], s_gjk[4][slot], s_gjk[5][slot]};
+                nrm = V3{s_gjk[6][slot], s_gjk[7][slot], s_gjk[8][slot]};
+                sd = s_gjk[9][slot];
+            }
+            gjk_hand_off(seg, it, live, ready, s, pa, pb, nrm, sd, box, e, queue, top, n1, lane);
+            return;
+        }
+    }
     const int stride = gridDim.x * blockDim.x;
     for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
         const int i = base + lane;
         const bool box = i < n_box;
-        bool manifold = false;
         int2 e = make_int2(0, 0);
+        NarrowItem it;
+        GjkSetup s;
+        bool live = false, ready = false;
+        V3 pa{0, 0, 0}, pb{0, 0, 0}, nrm{0, 0, 0};
+        float sd = 0.0f;
         if (i < n) {
             e = box ? queue[i] : queue[n1 - 1 - (i - n_box)];
-            NarrowItem it;
-            if (narrow_setup(m, seg, body_q, e, it)) {
-                V3 pa, pb, nrm;
-                manifold = gjk_stage(it.wr, it.ga, it.gb, pa, pb, nrm);
-                if (manifold) {
-                    float4* h = it.wr.slots + kSlotF4 - 3;
-                    h[0] = make_float4(pa.x, pa.y, pa.z, 0.0f);
-                    h[1] = make_float4(pb.x, pb.y, pb.z, 0.0f);
-                    h[2] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
-                } else {
-                    narrow_finish(seg, it);
-                }
-            }
+            live = narrow_setup(m, seg, body_q, e, it);
+            ready = live && gjk_prepare(it.ga, it.gb, s);
+            if (ready && !mpr_stage(s, pa, pb, nrm, sd)) gjk_core(s.p, 0.0f, pa, pb, nrm, sd);
         }
-        const unsigned below = (1u << lane) - 1u;
-        const unsigned bb = __ballot_sync(kFull, manifold && box);
-        const unsigned bo = __ballot_sync(kFull, manifold && !box);
-        int ob = 0, oo = 0;
-        if (lane == 0 && bb) ob = atomicAdd(&seg.work_counter[1], __popc(bb));
-        if (lane == 0 && bo) oo = atomicAdd(&seg.work_counter[7], __popc(bo));
-        ob = __shfl_sync(kFull, ob, 0);
-        oo = __shfl_sync(kFull, oo, 0);
-        if (manifold && box) queue[top - (ob + __popc(bb & below))] = e;
-        if (manifold && !box) queue[top - n1 + 1 + (oo + __popc(bo & below))] = e;
+        gjk_hand_off(seg, it, live, ready, s, pa, pb, nrm, sd, box, e, queue, top, n1, lane);
     }
 }
 
-__global__ void __launch_bounds__(kNT, kManifoldMinBlocks)
+template <int kMinBlocks>
+__global__ void __launch_bounds__(kNT, kMinBlocks)
 narrow_manifold_kernel(NbModelDesc m, const float* __restrict__ body_q, NbContactSeg seg) {
     const int n1 = seg.work_counter[3];
     int nb = seg.work_counter[1], no = seg.work_counter[7];
@@ -1146,7 +1206,7 @@ namespace {
 // drive several GPUs; the mutex orders first calls from several host threads).
 constexpr int kMaxCollideDevices = 64;
 struct NarrowOccupancy {
-    int analytic = 0, prefilter = 0, gjk = 0, manifold = 0;
+    int analytic = 0, prefilter = 0, gjk[2] = {0, 0}, manifold[2] = {0, 0};  // [few, many bodies]
 };
 std::mutex g_occ_mutex;
 NarrowOccupancy g_occ[kMaxCollideDevices];
@@ -1158,21 +1218,29 @@ cudaError_t narrow_occupancy(NarrowOccupancy* out) {
     if (dev < 0 || dev >= kMaxCollideDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(g_occ_mutex);
     NarrowOccupancy& c = g_occ[dev];
-    if (!c.gjk) {
+    if (!c.gjk[0]) {
         // default grids: one wave at each kernel's occupancy (grid-stride loops)
-        int a = 0, p = 0, g = 0, f = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, narrow_analytic_kernel, kNT, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, gjk_prefilter_kernel, kNT, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g, narrow_gjk_kernel, kNT, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, narrow_manifold_kernel, kNT, 0);
-        c.analytic = a > 0 ? a : 4;
-        c.prefilter = p > 0 ? p : 4;
-        c.gjk = g > 0 ? g : 4;
-        c.manifold = f > 0 ? f : 4;
+        auto blocks = [](auto kernel) {
+            int n = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kNT, 0);
+            return n > 0 ? n : 4;
+        };
+        c.analytic = blocks(narrow_analytic_kernel);
+        c.prefilter = blocks(gjk_prefilter_kernel);
+        c.manifold[0] = blocks(narrow_manifold_kernel<kManifoldBlocksFew>);
+        c.manifold[1] = blocks(narrow_manifold_kernel<kManifoldBlocksMany>);
+        c.gjk[1] = blocks(narrow_gjk_kernel<kGjkBlocksMany>);
+        c.gjk[0] = blocks(narrow_gjk_kernel<kGjkBlocksFew>);
     }
     *out = c;
     return cudaSuccess;
 }
+
+// A pile has about one MPR/GJK item per body (0.85 on 4096 landed worlds of mixed shapes): up to the
+// threads of the few-bodies variants they all run at once.  us, few / many variants without the sharing
+// below: one world of 64 boxes 127 / 131 (whole substep), 300 such worlds (two collides) 340 / 352, 1024
+// mixed worlds (two substeps) 652 / 668, 4096 mixed worlds (one collide) 566 / 510.
+bool narrow_is_small(const NbModelDesc* m, int sms) { return m->body_count <= sms * kGjkBlocksFew * kNT; }
 
 }  // namespace
 
@@ -1200,10 +1268,15 @@ cudaError_t nb_launch_collide(const NbModelDesc* m, const float* body_q, const N
     gjk_prefilter_kernel<<<grid > 0 ? grid : sms * occ.prefilter, kNT, 0, stream>>>(*m, *seg);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    narrow_gjk_kernel<<<grid > 0 ? grid : sms * occ.gjk, kNT, 0, stream>>>(*m, body_q, *seg);
+    const bool few = narrow_is_small(m, sms);
+    const int gjk = grid > 0 ? grid : sms * occ.gjk[few ? 0 : 1];
+    if (few) narrow_gjk_kernel<kGjkBlocksFew><<<gjk, kNT, 0, stream>>>(*m, body_q, *seg);
+    else narrow_gjk_kernel<kGjkBlocksMany><<<gjk, kNT, 0, stream>>>(*m, body_q, *seg);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    narrow_manifold_kernel<<<grid > 0 ? grid : sms * occ.manifold, kNT, 0, stream>>>(*m, body_q, *seg);
+    const int manifold = grid > 0 ? grid : sms * occ.manifold[few ? 0 : 1];
+    if (few) narrow_manifold_kernel<kManifoldBlocksFew><<<manifold, kNT, 0, stream>>>(*m, body_q, *seg);
+    else narrow_manifold_kernel<kManifoldBlocksMany><<<manifold, kNT, 0, stream>>>(*m, body_q, *seg);
     return cudaGetLastError();
 }
 

@@ -1118,46 +1118,41 @@ NB_D bool gjk_prepare(const Geom& ga, const Geom& gb, GjkSetup& s) {
     return true;
 }
 
-// MPR, then GJK when MPR finds no overlap.  Returns true when the pair still
-// needs its manifold (build_manifold from the returned witness points and
-// normal, in the pair's relative frame); false when it is finished -- rejected
-// early, or its single contact (spheres, or a distance beyond the threshold)
-// already written.
-__device__ __noinline__ bool gjk_stage(Writer& w, const Geom& ga, const Geom& gb, V3& point_a, V3& point_b,
-                                       V3& normal) {
-    GjkSetup s;
-    if (!gjk_prepare(ga, gb, s)) return false;
-    float pen, sd;
-    bool collision = mpr_core(s.p, s.enlarge, point_a, point_b, normal, pen);
-    if (collision) {
-        sd = -pen + s.enlarge;
-        float he = s.enlarge * 0.5f;
-        point_a = sub(point_a, mul(normal, he));
-        point_b = add(point_b, mul(normal, he));
-    } else {
-        gjk_core(s.p, 0.0f, point_a, point_b, normal, sd);
-    }
-    if (s.skip_multi || sd > s.threshold) {
-        V3 pt = smul(0.5f, add(point_a, point_b));
-        pt = add(qrot(s.qa, pt), s.pa);
-        V3 nws = qrot(s.qa, normal);
-        ContactData cd = s.tmpl;
-        cd.center = pt;
-        cd.normal = nws;
-        cd.dist = sd;
-        cd.sub_key = s.tmpl.sub_key << 3;
-        post_process(cd, s.p.a.type, s.p.b.type);
-        write_contact(w, cd, true);
-        return false;
-    }
+// What MPR makes of a pair: true when it finds an overlap, with the witness points, normal and signed
+// distance taken back to the shapes' own surfaces.
+NB_D bool mpr_stage(const GjkSetup& s, V3& point_a, V3& point_b, V3& normal, float& sd) {
+    float pen;
+    if (!mpr_core(s.p, s.enlarge, point_a, point_b, normal, pen)) return false;
+    sd = -pen + s.enlarge;
+    float he = s.enlarge * 0.5f;
+    point_a = sub(point_a, mul(normal, he));
+    point_b = add(point_b, mul(normal, he));
     return true;
 }
 
-// the manifold of a pair gjk_stage left unfinished, from its witness points and normal
+// The pair's single contact, if it has one (spheres, or a distance beyond the threshold).  Returns true
+// when the pair needs its manifold instead (build_manifold from the witness points and normal, in the
+// pair's relative frame).
+NB_D bool gjk_finish(Writer& w, const GjkSetup& s, V3 point_a, V3 point_b, V3 normal, float sd) {
+    if (!(s.skip_multi || sd > s.threshold)) return true;
+    V3 pt = smul(0.5f, add(point_a, point_b));
+    pt = add(qrot(s.qa, pt), s.pa);
+    V3 nws = qrot(s.qa, normal);
+    ContactData cd = s.tmpl;
+    cd.center = pt;
+    cd.normal = nws;
+    cd.dist = sd;
+    cd.sub_key = s.tmpl.sub_key << 3;
+    post_process(cd, s.p.a.type, s.p.b.type);
+    write_contact(w, cd, true);
+    return false;
+}
+
+// the manifold of a pair gjk_finish left unfinished, from its witness points and normal
 __device__ __noinline__ void gjk_manifold(Writer& w, const Geom& ga, const Geom& gb, V3 point_a, V3 point_b,
                                           V3 normal) {
     GjkSetup s;
-    if (!gjk_prepare(ga, gb, s)) return;  // never: the stage passed the same test
+    if (!gjk_prepare(ga, gb, s)) return;  // never: the pair passed the same test before
     build_manifold(w, s.p, s.qa, s.pa, point_a, point_b, normal, s.tmpl);
 }
 
