@@ -999,6 +999,7 @@ __device__ __forceinline__ void adjoint_contacts(const NbModelDesc& m, const NbX
     const float* S_it = io.tape_state + (size_t)it * B * 13;
     int n = io.active_count[it];
     n = n < io.active_capacity ? n : io.active_capacity;
+    constexpr bool kOnlyA = (kChunk + 1) * kDirs <= 10, kOnlyB = kChunk * kDirs >= 10;  // whose inputs the chunk holds
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const int rec = io.active[2 * ((size_t)it * io.active_capacity + e)];
         const int w = io.active[2 * ((size_t)it * io.active_capacity + e) + 1];
@@ -1007,6 +1008,8 @@ __device__ __forceinline__ void adjoint_contacts(const NbModelDesc& m, const NbX
         const ContactC c = load_contact(m, r, b0, S_it);
         const bool dyn_a = c.la >= 0 && !c.kin_a, dyn_b = c.lb >= 0 && !c.kin_b;
         if (!dyn_a && !dyn_b) continue;
+        // a chunk of one body's inputs has nothing to add where that body does not move
+        if ((kOnlyB && !dyn_b) || (kOnlyA && kChunk > 0 && !dyn_a)) continue;
         float sa[13], sb[13];
         side_state(S_it, b0, c.la, sa);
         side_state(S_it, b0, c.lb, sb);
@@ -1038,10 +1041,12 @@ __device__ __forceinline__ void adjoint_contacts(const NbModelDesc& m, const NbX
 
 // One block row per chunk: a contact's chunks, each a pass over the whole contact with dual numbers, run
 // on kChunks threads at once instead of one after another.  Bound by that chain: with some 20,000 active
-// contacts one thread per contact is one warp per scheduler (256 stacks of 16 boxes: 46 us per launch; in chunks of four
-// directions 31, of two 40).
-__global__ void __launch_bounds__(kThreads) adjoint_contacts_kernel(NbModelDesc m, NbXpbdParams p, NbAdjointIO io,
-                                                                    NbContactSeg seg, int it, float dt) {
+// contacts one thread per contact is one warp per scheduler.  256 stacks of 16 boxes, us per launch: 46 in
+// one thread, 31 in chunks of four directions, 40 of two; 27 with three CTAs per SM (168 registers) in
+// place of two.
+__global__ void __launch_bounds__(kThreads, 3) adjoint_contacts_kernel(NbModelDesc m, NbXpbdParams p,
+                                                                       NbAdjointIO io, NbContactSeg seg, int it,
+                                                                       float dt) {
     static_assert(kChunks == 5, "one case per chunk");
     switch (blockIdx.y) {
         case 0: return adjoint_contacts<0>(m, p, io, seg, it, dt);
