@@ -67,3 +67,28 @@ def test_default_schedule_by_world_count():
     # 32 threads cannot hold 200 bodies: the smallest group that does
     assert default_mode(200, 5000, sms) == ("groups_compact", 64)
     assert default_mode(600, 5000, sms) == ("batch", None)
+
+
+@pytest.mark.parametrize("grid", [1, 2, 7])
+def test_narrow_phase_with_few_ctas(cuda, grid):
+    """More queue items than threads: the analytic kernel's ordered tiles and the MPR/GJK kernel's loop give
+    the contacts of the default grids, where every item has a thread (or two)."""
+    import ctypes as C
+
+    model, info = scenes.scene_c2(seed=21, worlds=24, nmin=8, nmax=90, device=cuda)
+    pipe, solver = CollisionPipeline(model), SolverXPBD(model, iterations=4)
+    a, b, want, got = model.state(), model.state(), pipe.contacts(), pipe.contacts()
+    for _ in range(12 * info["substeps"]):
+        pipe.collide(a, want)
+        solver.step(a, b, None, want, info["dt"] / info["substeps"])
+        a, b = b, a
+    pipe.collide(a, want)
+    lib, desc, stream = _lib.load(), pipe.desc(), C.c_void_p(_lib.stream_handle(model.device))
+    seg, pub = pipe.seg_struct(got), pipe.public_struct(got)
+    _lib.check("nb_collide", lib.nb_collide(C.byref(desc), C.c_void_p(a.body_q.data_ptr()), C.byref(seg), grid, stream))
+    _lib.check("nb_publish_contacts", lib.nb_publish_contacts(C.byref(desc), C.byref(seg), C.byref(pub), stream))
+    n = int(want.rigid_contact_count.item())
+    assert n > 128 * grid and int(got.rigid_contact_count.item()) == n and pipe.status(got) == 0
+    for k in ("shape0", "shape1", "point0", "point1", "offset0", "offset1", "normal", "margin0", "margin1"):
+        x, y = getattr(want, f"rigid_contact_{k}")[:n], getattr(got, f"rigid_contact_{k}")[:n]
+        assert torch.equal(x, y), k
