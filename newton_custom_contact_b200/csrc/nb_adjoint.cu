@@ -907,13 +907,18 @@ __global__ void __launch_bounds__(kThreads) adjoint_forward_kernel(NbModelDesc m
             d12[0] = la.x; d12[1] = la.y; d12[2] = la.z; d12[3] = aa.x; d12[4] = aa.y; d12[5] = aa.z;
             d12[6] = lb.x; d12[7] = lb.y; d12[8] = lb.z; d12[9] = ab.x; d12[10] = ab.y; d12[11] = ab.z;
         };
-        auto add = [&](int i, int, const float* d6) {
+        auto load = [&](int i, float* a6) {
+            const float* acc = io.delta_acc + 6 * (size_t)(b0 + i);
+#pragma unroll
+            for (int q = 0; q < 6; ++q) a6[q] = acc[q];
+        };
+        auto store = [&](int i, const float* a6, int n) {
             float* acc = io.delta_acc + 6 * (size_t)(b0 + i);
 #pragma unroll
-            for (int q = 0; q < 6; ++q) acc[q] = acc[q] + d6[q];
-            if (weighting) io.count_acc[b0 + i] += 1;
+            for (int q = 0; q < 6; ++q) acc[q] = a6[q];
+            if (weighting) io.count_acc[b0 + i] += n;
         };
-        nb::ordered_pass<kThreads, kThreads>(s_batch, nc, 0, t, test, solve, add);
+        nb::ordered_pass<kThreads, kThreads>(s_batch, nc, nb, 0, t, test, solve, load, store);
         __syncthreads();
         for (int i = t; i < nb; i += kThreads) {
             const int bi = b0 + i;

@@ -113,11 +113,14 @@ struct SBodiesT {
         }
         return r;
     }
-    // the reference's atomic_add(deltas, i, spatial_vector(lin, ang)): old + value, per component
-    // (only body i's owner thread of the ordered pass calls this)
-    __device__ __forceinline__ void add(int i, const float* d6) {
+    // body i's accumulator (only its owner thread of the ordered pass calls these)
+    __device__ __forceinline__ void load_acc(int i, float* a6) const {
 #pragma unroll
-        for (int k = 0; k < 6; ++k) acc[k * nb + i] = acc[k * nb + i] + d6[k];
+        for (int k = 0; k < 6; ++k) a6[k] = acc[k * nb + i];
+    }
+    __device__ __forceinline__ void store_acc(int i, const float* a6) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) acc[k * nb + i] = a6[k];
     }
     // read and clear the accumulated delta of body i; false when nothing was added
     __device__ bool take(int i, V3& lin, V3& ang) {
@@ -613,8 +616,9 @@ __device__ void joint_axes(const NbModelDesc& m, int start, int count, const flo
 // the parent (side A) and child (side B) bodies.
 template <class SB>
 __device__ __forceinline__ bool joint_active(const NbModelDesc& m, const SB& S, int b0, int j, int& ends) {
-    if (!m.joint_enabled[j] || m.joint_type[j] == NB_JOINT_FREE) return false;
-    const int id_c = m.joint_child[j], id_p = m.joint_parent[j];
+    // four loads at once: every iteration waits for them
+    const int enabled = m.joint_enabled[j], type = m.joint_type[j], id_c = m.joint_child[j], id_p = m.joint_parent[j];
+    if (!enabled || type == NB_JOINT_FREE) return false;
     const int lc = id_c - b0, lp = id_p < 0 ? -1 : id_p - b0;
     if ((id_p < 0 || S.inv_m(lp) == 0.0f) && S.inv_m(lc) == 0.0f) return false;
     ends = nb::ends_pack(lp, lc);
@@ -866,7 +870,7 @@ __device__ void joint_forces(const NbModelDesc& m, SB& S, int b0, int j0, int j1
 // record order (nb_ordered.cuh); with weighting, the owner also counts them
 // (the reference's contact_inv_weight).  imp_scratch (optional) receives each
 // active record's A-side delta.
-template <int G, class SB>
+template <int G, bool kLean, class SB>
 __device__ __forceinline__ void contact_pass(const NbModelDesc& m, SB& S, const float4* __restrict__ R, int nc,
                                              Batch<G>& B, int g, int t, float relaxation, float dt, bool weighting,
                                              float* imp_scratch) {
@@ -879,11 +883,14 @@ __device__ __forceinline__ void contact_pass(const NbModelDesc& m, SB& S, const 
         solve_contact(m, S, r[0], r[1], r[2], r[3], r[4], relaxation, dt, d12,
                       imp_scratch ? imp_scratch + (size_t)k * 6 : nullptr);
     };
-    auto add = [&](int i, int, const float* d6) {
-        S.add(i, d6);
-        if (weighting) S.cnt[i] += 1;
+    auto load = [&](int i, float* a6) { S.load_acc(i, a6); };
+    auto store = [&](int i, const float* a6, int n) {
+        S.store_acc(i, a6);
+        if (weighting) S.cnt[i] += n;
     };
-    nb::ordered_pass<G, kST>(B, nc, g, t, test, solve, add);
+    // the full kernels are short of registers: their owners add in shared memory (256 arms: 172 us per
+    // step with the sums in registers, 156 without)
+    nb::ordered_pass<G, kST>(B, nc, kLean ? S.nb : nb::kManyBodies, g, t, test, solve, load, store);
 }
 
 // world's largest penetration max(-d, 0) over its contacts (group reduction
@@ -977,8 +984,9 @@ __device__ __forceinline__ void warm_start(const NbModelDesc& m, const NbStepIO&
         d12[0] = L.x; d12[1] = L.y; d12[2] = L.z; d12[3] = aa.x; d12[4] = aa.y; d12[5] = aa.z;
         d12[6] = Lb.x; d12[7] = Lb.y; d12[8] = Lb.z; d12[9] = ab.x; d12[10] = ab.y; d12[11] = ab.z;
     };
-    auto add_row = [&](int i, int, const float* d6) { S.add(i, d6); };
-    nb::ordered_pass<G, kST>(B, nc, g, t, test, solve, add_row);
+    auto load = [&](int i, float* a6) { S.load_acc(i, a6); };
+    auto store = [&](int i, const float* a6, int) { S.store_acc(i, a6); };
+    nb::ordered_pass<G, kST>(B, nc, nb::kManyBodies, g, t, test, solve, load, store);
     group_sync<G>(g);
     for (int i = t; i < nb; i += G) {
         V3 dl, da;
@@ -1170,10 +1178,9 @@ __device__ __forceinline__ void step_world(const NbModelDesc& m, const NbXpbdPar
     if constexpr (kWarm) {
         if (has_contacts && io.ws_lambda) warm_start<G>(m, io, seg, S, R, nc, rec_base, b0, g, t, pen_slot, B, dt);
     }
-    const V3 zero3{0.0f, 0.0f, 0.0f};
     for (int it = 0; it < p.iterations; ++it) {
         if (has_contacts) {
-            contact_pass<G>(m, S, R, nc, B, g, t, p.rigid_contact_relaxation, dt, weighting,
+            contact_pass<G, kLean>(m, S, R, nc, B, g, t, p.rigid_contact_relaxation, dt, weighting,
                             want_imp ? io.impulse_scratch + (size_t)rec_base * 6 : nullptr);
             if constexpr (!kLean || kImp) {
                 if (want_imp) {
@@ -1213,8 +1220,9 @@ __device__ __forceinline__ void step_world(const NbModelDesc& m, const NbXpbdPar
                     auto jsolve = [&](int k, float* d12) {
                         solve_joint(m, S, b0, j0 + k, io.joint_target_pos, io.joint_target_vel, p, dt, d12, jimp);
                     };
-                    auto jadd = [&](int i, int, const float* d6) { S.add(i, d6); };
-                    nb::ordered_pass<G, kST>(B, j1 - j0, g, t, jtest, jsolve, jadd);
+                    auto jload = [&](int i, float* a6) { S.load_acc(i, a6); };
+                    auto jstore = [&](int i, const float* a6, int) { S.store_acc(i, a6); };
+                    nb::ordered_pass<G, kST>(B, j1 - j0, nb::kManyBodies, g, t, jtest, jsolve, jload, jstore);
                 }
             }
             for (int i = t; i < nb; i += G) {
@@ -1240,8 +1248,9 @@ __device__ __forceinline__ void step_world(const NbModelDesc& m, const NbXpbdPar
                 int ends;
                 restitution_contact(m, S, R + (size_t)k * 5, b0, io.body_q_in, io.body_qd_in, dt, d12, ends);
             };
-            auto radd = [&](int i, int, const float* d6) { S.add(i, d6); };
-            nb::ordered_pass<G, kST>(B, nc, g, t, rtest, rsolve, radd);
+            auto rload = [&](int i, float* a6) { S.load_acc(i, a6); };
+            auto rstore = [&](int i, const float* a6, int) { S.store_acc(i, a6); };
+            nb::ordered_pass<G, kST>(B, nc, nb::kManyBodies, g, t, rtest, rsolve, rload, rstore);
             // apply_body_delta_velocities (kernels.py:881-887) over every body
             for (int i = t; i < nb; i += G) {
                 V3 dl, da;
