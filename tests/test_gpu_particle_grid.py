@@ -52,7 +52,7 @@ def _compare(model, grid_size=None, iterations=3, dt=1.0 / 240.0):
         assert np.array_equal(got, np.ascontiguousarray(want[act], np.float32).view(np.uint32))
 
 
-@pytest.mark.parametrize("count", [2, 7, 8, 9, 31, 64, 1023, 1024, 1025, 2500])
+@pytest.mark.parametrize("count", [2, 7, 8, 9, 31, 64, 1023, 1024, 1025, 2500, 4096, 4097])
 def test_counts_at_the_bucket_edges(cuda, count):
     # about 4 particles per cell of 42 mm
     _compare(_cloud(count, 0.5 * 0.026 * count ** (1.0 / 3.0), (0.1, -0.2, 0.3), count, cuda=cuda))
