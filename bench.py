@@ -512,9 +512,9 @@ def particles_arm(dev, stream, flush, steps, warmup):
             "soft_contacts_at_step_end": int(torch.stack(contacts_seen).float().mean().item()),
             "min_height_above_radius_m": float((q[act, 2] - r[act]).min().item()),
             "final_state_finite": bool(torch.isfinite(q).all().item()),
-            # soft contacts 3 kernels, integrate 1, then constraints (+ bending) + apply per iteration
+            # soft contacts 3 kernels, integrate 1, then ranges, scatter, constraints (+ bending), apply per iteration
             "status": solver._particles.status(),
-            "gpu_launches_per_substep": 3 + 1 + (3 if model.edge_count else 2) * 8, "bending_edges": model.edge_count,
+            "gpu_launches_per_substep": 3 + 1 + (5 if model.edge_count else 4) * 8, "bending_edges": model.edge_count,
             "scene_build_s": round(build_s, 1)}
 
 

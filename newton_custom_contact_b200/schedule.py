@@ -97,12 +97,12 @@ def default_mode(max_world_bodies: int, world_count: int, sms: int | None = None
     8..32 bodies):
 
         worlds   8..128 bodies            8..32 bodies
-        37        59 /  70 /  94 / 135     57 /  61 /  65 /  69
-        150       64 /  79 / 104 / 159     57 /  62 /  66 /  72
-        600      146 /  97 / 118 / 189    130 /  88 /  78 /  84
-        1024     213 / 138 / 119 / 191    192 / 115 /  79 /  89
-        1600     318 / 205 / 155 / 203    285 / 170 / 111 /  95
-        4096     817 / 521 / 361 / 304    682 / 410 / 240 / 159
+        37        56 /  73 /  87 / 126     56 /  59 /  62 /  66
+        150       63 /  78 / 100 / 148     58 /  60 /  62 /  70
+        600      147 /  97 / 111 / 163    133 /  87 /  68 /  81
+        1024     212 / 135 / 114 / 175    194 / 110 /  69 /  86
+        1600     317 / 199 / 148 / 188    287 / 164 / 106 /  89
+        4096     805 / 510 / 343 / 280    684 / 396 / 223 / 153
 
     Within the group modes the full slab is taken where it fits a group's share, else the compact one
     (they differ by a few percent); 256 threads and worlds beyond every share run as batches."""
