@@ -374,8 +374,8 @@ class CollisionPipeline:
 
     def set_step_schedule(self, group_threads: int | None = None, mode: str | None = None) -> None:
         """Choose how the step kernel maps worlds to thread groups (see schedule.py):
-        ``mode`` "groups", "groups_compact" or "batch", with ``group_threads``; default: the
-        smallest independent group whose arena share holds the largest world, else batches."""
+        ``mode`` "groups", "groups_compact" or "batch", with ``group_threads``; default: by
+        world count and size (schedule.default_mode)."""
         from .schedule import build_schedule
 
         sched = build_schedule(self.model, group_threads, mode)

@@ -12,8 +12,8 @@ Two ways to map worlds to the GPU:
 * batch mode: one world per thread group of G threads (G = 32: a warp per
   world ... G = 256: a CTA per world); a CTA holds 256 / G groups that share
   one arena.  Worlds are packed, largest first, into batches that fit one
-  arena; CTAs pull batches from a device counter.  Used for worlds too large
-  for a warp's share.
+  arena; CTAs pull batches from a device counter.  Used with a CTA per world
+  when the worlds are few, and for worlds too large for a group's share.
 
 ``autotune`` times the candidate schedules on the caller's own scene and
 keeps the fastest; results are cached per world-size histogram.
