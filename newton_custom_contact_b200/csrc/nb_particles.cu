@@ -379,7 +379,7 @@ struct GroupScratch {
         float c[NB_PARTICLE_MAX_NEIGHBORS][3];     // the accepted neighbours' contributions, in ascending index
     };
     int j[NB_PARTICLE_MAX_NEIGHBORS];              // accepted neighbours
-    int nm, n;                                     // candidates listed, neighbours accepted
+    int n;                                         // neighbours accepted
 };
 
 template <bool kSorted>
@@ -395,6 +395,7 @@ particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io, NbSoftContacts s
     }
     const int lane = threadIdx.x & (kGroup - 1);
     const unsigned gmask = ((1u << kGroup) - 1u) << (threadIdx.x & 31 & ~(kGroup - 1));
+    const unsigned below = (1u << (threadIdx.x & 31)) - 1u;  // the lanes before this one
     GroupScratch& G = s_group[threadIdx.x / kGroup];
     int i = blockIdx.x * kSlots + threadIdx.x / kGroup;
     if constexpr (kSorted) {
@@ -411,7 +412,7 @@ particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io, NbSoftContacts s
     const int spring_hi = pd.spring_count > 0 ? pd.particle_spring_start[i + 1] : 0;
     const int soft_lo = has_sc ? sc.particle_start[i] : 0;
     const int soft_hi = has_sc ? min(sc.particle_start[i + 1], min(sc.max, sc.count[0])) : 0;
-    if (lane == 0) G.nm = G.n = 0;
+    if (lane == 0) G.n = 0;
     __syncwarp(gmask);
 
     if (g.on) {
@@ -475,11 +476,12 @@ particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io, NbSoftContacts s
                     if (lane >= o) run += y;
                 }
                 const int total = __shfl_sync(gmask, run, kGroup - 1, kGroup);
+                if (total <= 0) continue;
                 run -= tot;
                 G.seg[2 * lane] = make_int4(beg - run, run + len, (int)key, r);
                 G.seg[2 * lane + 1] = make_int4(beg2 - run - len, run + tot, (int)key, r);
                 __syncwarp(gmask);
-                int q = 0;
+                int q = 0, nm = 0;  // nm: candidates listed, the same number in every lane
                 int4 seg = G.seg[0];
                 for (int base = 0; base < total; base += kAhead * kGroup) {
                     int2 en[kAhead];
@@ -507,17 +509,19 @@ particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io, NbSoftContacts s
                         const int dx = (int)((w - mine) << 22) >> 22;
                         const int dy = (int)(((w >> 10) - (mine >> 10)) << 22) >> 22;
                         const int dz = (int)(((w >> 20) - (mine >> 20)) << 22) >> 22;
-                        if (en[u].y != i && ((w ^ row_key[u]) & 0x300C0000u) == 0u && dx * dx + dy * dy + dz * dz <= r2)
-                            G.maybe[atomicAdd(&G.nm, 1)] = en[u].y;
+                        const bool keep = en[u].y != i && ((w ^ row_key[u]) & 0x300C0000u) == 0u &&
+                                          dx * dx + dy * dy + dz * dz <= r2;
+                        const unsigned kept = __ballot_sync(gmask, keep) & gmask;
+                        if (keep) G.maybe[nm + __popc(kept & below)] = en[u].y;
+                        nm += __popc(kept);
                     }
-                    __syncwarp(gmask);
-                    // the list is tested when another round might not fit, and at the end
-                    const int nm = G.nm;
+                    // the list is tested when another round might not fit, and at the end; every lane counts
+                    // it from the ballots, so that the whole group comes here or goes on to the next round
                     if (nm > kMaybe - kAhead * kGroup || base + kAhead * kGroup >= total) {
+                        __syncwarp(gmask);  // the list is visible
                         for (int a = lane; a < nm; a += kGroup) consider(G.maybe[a]);
-                        __syncwarp(gmask);
-                        if (lane == 0) G.nm = 0;
-                        __syncwarp(gmask);
+                        __syncwarp(gmask);  // ... and read
+                        nm = 0;
                     }
                 }
             }

@@ -80,3 +80,20 @@ def test_one_large_among_small_particles(cuda):
 def test_small_scratch_takes_the_lists(cuda, grid_size):
     # 900 particles: sorted from 2048 (ranges and entries fit), linked lists below
     _compare(_cloud(900, 0.13, (0.0, 0.0, 0.0), 9, cuda=cuda), grid_size=grid_size)
+
+
+@pytest.mark.parametrize("count", [900, 2300, 4500])
+def test_many_candidates_within_reach(cuda, count):
+    # small particles beside one large one: dozens to hundreds of candidates of a particle pass the packed distance,
+    # so the list of candidates fills and is tested several times, at every phase of its rounds
+    model = _cloud(count, 0.09, (0.02, -0.03, 0.05), count, radii=(0.001, 0.0025), cuda=cuda)
+    h, h_q = model.host("particle_radius"), model.host("particle_q")
+    h[7] = 0.05
+    h_q[7] = (0.7, 0.7, 0.7)  # away from the cloud: its own contacts would exceed the neighbour limit
+    model.particle_radius.copy_(torch.from_numpy(h))
+    model.particle_q.copy_(torch.from_numpy(h_q))
+    model.particle_max_radius = 0.05
+    reach = h[0] + model.particle_max_radius + model.particle_cohesion
+    near = np.linalg.norm(h_q[:, None] - h_q[None, :200], axis=2) < reach
+    assert near.sum(axis=0).max() > 64
+    _compare(model)
