@@ -263,6 +263,13 @@ NB_D uint32_t pack_axis(float x, float inv_h) {
 NB_D uint32_t pack_pos(V3 x, float inv_h) {
     return pack_axis(x.x, inv_h) | (pack_axis(x.y, inv_h) << 10) | (pack_axis(x.z, inv_h) << 20);
 }
+// An entry's first word: the packed position, with kLargeEntry set for a particle beyond the model's
+// particle_max_radius (a program may change radii later): it may touch particles whose reach, which counts on
+// that radius, ends before it.
+constexpr uint32_t kLargeEntry = 1u << 30;
+NB_D uint32_t entry_word(const NbParticleDesc& pd, int p, V3 x, float inv_h) {
+    return pack_pos(x, inv_h) | (pd.particle_radius[p] > pd.particle_max_radius ? kLargeEntry : 0u);
+}
 NB_D void grid_insert(const Grid& g, int table, int p, V3 x) {
     const uint32_t b = cell_hash(cell_of(x.x, g.inv_h), cell_of(x.y, g.inv_h), cell_of(x.z, g.inv_h), g.mask);
     if (g.sorted) atomicAdd(&g.count[b], 1);
@@ -317,7 +324,7 @@ __global__ void __launch_bounds__(kThreads) particle_scatter_kernel(NbParticleDe
     const V3 x = ld3(xq, p);
     const uint32_t b = cell_hash(cell_of(x.x, g.inv_h), cell_of(x.y, g.inv_h), cell_of(x.z, g.inv_h), g.mask);
     const int at = g.range[b].x + atomicSub(&g.count[b], 1) - 1;
-    g.entry[at] = make_int2((int)pack_pos(x, g.inv_h), p);
+    g.entry[at] = make_int2((int)entry_word(pd, p, x, g.inv_h), p);
 }
 
 // integrate_particles (newton/_src/solvers/solver.py:11-47): semi-implicit Euler, gravity on
@@ -441,7 +448,7 @@ particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io, NbSoftContacts s
         if constexpr (kSorted) {
             // squared reach in the packed positions' units: a packed difference is off by less than 1 per
             // axis, and by the rounding of x * inv_h far from the origin; past half the packed period
-            // nothing is rejected
+            // nothing is rejected, nor is a particle larger than the reach counts on
             const float far = fmaxf(fabsf(x.x), fmaxf(fabsf(x.y), fabsf(x.z))) + reach;
             const float ru = (reach * 256.0f + far * 1.0e-4f) * g.inv_h + 2.0f;
             const int r2 = ru < 500.0f ? (int)(ru * ru) + 1 : 0x7fffffff;
@@ -510,7 +517,7 @@ particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io, NbSoftContacts s
                         const int dy = (int)(((w >> 10) - (mine >> 10)) << 22) >> 22;
                         const int dz = (int)(((w >> 20) - (mine >> 20)) << 22) >> 22;
                         const bool keep = en[u].y != i && ((w ^ row_key[u]) & 0x300C0000u) == 0u &&
-                                          dx * dx + dy * dy + dz * dz <= r2;
+                                          (dx * dx + dy * dy + dz * dz <= r2 || (w & kLargeEntry) != 0u);
                         const unsigned kept = __ballot_sync(gmask, keep) & gmask;
                         if (keep) G.maybe[nm + __popc(kept & below)] = en[u].y;
                         nm += __popc(kept);
@@ -856,7 +863,7 @@ __global__ void __launch_bounds__(1024) particle_regrid_kernel(NbParticleDesc pd
     for (int b = t; b < M; b += kT) s_count[b] = 0;
     __syncthreads();
     int bucket[kPer], rank[kPer];
-    uint32_t packed[kPer];
+    uint32_t word[kPer];
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
         const int p = t + k * kT;
@@ -864,7 +871,7 @@ __global__ void __launch_bounds__(1024) particle_regrid_kernel(NbParticleDesc pd
         if (p >= pd.particle_count || !active(pd, p)) continue;
         const V3 x = apply ? apply_delta(pd, io, dt, p) : ld3(io.particle_q_out, p);
         bucket[k] = (int)cell_hash(cell_of(x.x, g.inv_h), cell_of(x.y, g.inv_h), cell_of(x.z, g.inv_h), g.mask);
-        packed[k] = pack_pos(x, g.inv_h);
+        word[k] = entry_word(pd, p, x, g.inv_h);
         rank[k] = atomicAdd(&s_count[bucket[k]], 1);
     }
     __syncthreads();
@@ -907,7 +914,7 @@ __global__ void __launch_bounds__(1024) particle_regrid_kernel(NbParticleDesc pd
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kPer; ++k)
-        if (bucket[k] >= 0) g.entry[s_count[bucket[k]] + rank[k]] = make_int2((int)packed[k], t + k * kT);
+        if (bucket[k] >= 0) g.entry[s_count[bucket[k]] + rank[k]] = make_int2((int)word[k], t + k * kT);
 }
 
 // apply_particle_shape_restitution (kernels.py:34-112) for static shapes: contacts tested at the

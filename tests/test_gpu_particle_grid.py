@@ -97,3 +97,47 @@ def test_many_candidates_within_reach(cuda, count):
     near = np.linalg.norm(h_q[:, None] - h_q[None, :200], axis=2) < reach
     assert near.sum(axis=0).max() > 64
     _compare(model)
+
+
+def _rows(rows, cuda):
+    """A model without gravity of (position, radius) rows: mass 0.02, particle_max_radius 0.02 and cohesion
+    2 mm, so cells of 42 mm, whatever the rows' radii."""
+    b = ModelBuilder(gravity=0.0)
+    for p, r in rows:
+        b.add_particle(tuple(float(c) for c in p), (0.0, 0.0, 0.0), 0.02, radius=r)
+    model = b.finalize(device=cuda)
+    model.particle_max_radius = 0.02
+    model.particle_cohesion = 0.002
+    return model
+
+
+@pytest.mark.parametrize("pairs", [12, 2100])  # one block's grid, and the three kernels'
+def test_neighbour_radius_beyond_the_maximum(cuda, pairs):
+    # Each pair lies in one cell, overlapping by 4 mm, with the large particle outside of the small one's
+    # reach by particle_max_radius: a candidate of its cell all the same
+    rows = []
+    for k in range(pairs):
+        o = 0.042 * 5.0 * np.array([k % 13, (k // 13) % 13, k // 169])
+        rows += [(o + (0.008, 0.021, 0.021), 0.002), (o + (0.036, 0.021, 0.021), 0.03)]
+    _compare(_rows(rows, cuda), iterations=2)
+
+
+def test_own_radius_beyond_the_maximum(cuda):
+    # Reach 2.4 cells around a cell's middle: five cells per axis, two rounds of rows, candidates told
+    # apart by their cells.  The small particles do not see the large one, so only its own correction is
+    # the oracle's.
+    rng = np.random.default_rng(2)
+    d = rng.normal(size=(24, 3))
+    d *= (rng.uniform(0.05, 0.08, 24) / np.linalg.norm(d, axis=1))[:, None]
+    d = np.concatenate([d, 0.08 * np.eye(3), -0.08 * np.eye(3)])  # cells 2 and -2
+    far = rng.uniform(-0.2, 0.2, (200, 3))
+    far = far[np.linalg.norm(far, axis=1) > 0.09]
+    model = _rows([((0.021, 0.021, 0.021), 0.08)] + [(0.021 + p, 0.002) for p in d] +
+                  [(0.021 + p, 0.0005) for p in far], cuda)
+    solver, a, b = SolverXPBD(model, iterations=1), model.state(), model.state()
+    solver.step(a, b, contacts=CollisionPipeline(model).contacts(), control=None, dt=1.0 / 240.0)
+    q, qd = model.host("particle_q"), model.host("particle_qd")
+    none = op.soft_collide(model._host, q, None, 0.01, 0)
+    want = op.step(model._host, particles.params(model), q, qd, None, none, 1.0 / 240.0, 1, 0.9, False)[0][0]
+    assert solver._particles.status() == 0 and not np.array_equal(want, q[0])
+    assert np.array_equal(b.particle_q[0].cpu().numpy().view(np.uint32), want.astype(np.float32).view(np.uint32))
