@@ -251,6 +251,11 @@ constexpr int kSmallParticles = 4096;  // most particles (and buckets) one block
 constexpr int kMinSorted = 8;        // fewest buckets of the sorted form: a row of 5 cells never wraps onto itself
 
 NB_D int cell_of(float x, float inv_h) { return (int)floorf(x * inv_h); }
+// the last of the cells searched from `first` on: at most 5, which keeps the loops bounded whatever the
+// scale, and none past the largest int, where far positions end up
+NB_D int last_cell(float x, float inv_h, int first) {
+    return min(cell_of(x, inv_h), first < INT32_MAX - 4 ? first + 4 : INT32_MAX);
+}
 NB_D uint32_t cell_hash(int cx, int cy, int cz, uint32_t mask) {
     return ((uint32_t)cx + (uint32_t)cy * 0x9E3779B1u + (uint32_t)cz * 0x85EBCA77u) & mask;
 }
@@ -424,11 +429,10 @@ particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io, NbSoftContacts s
 
     if (g.on) {
         const float reach = (radius + pd.particle_max_radius + pd.particle_cohesion) * 1.001f + 1.0e-6f;
-        // the reach is at most ~1 cell (cell size 2 * max radius + cohesion), so a span of 3 cells per axis;
-        // the cap keeps the loops bounded whatever the scale
-        const int x0 = cell_of(x.x - reach, g.inv_h), x1 = min(cell_of(x.x + reach, g.inv_h), x0 + 4);
-        const int y0 = cell_of(x.y - reach, g.inv_h), y1 = min(cell_of(x.y + reach, g.inv_h), y0 + 4);
-        const int z0 = cell_of(x.z - reach, g.inv_h), z1 = min(cell_of(x.z + reach, g.inv_h), z0 + 4);
+        // the reach is at most ~1 cell (cell size 2 * max radius + cohesion), so a span of 3 cells per axis
+        const int x0 = cell_of(x.x - reach, g.inv_h), x1 = last_cell(x.x + reach, g.inv_h, x0);
+        const int y0 = cell_of(x.y - reach, g.inv_h), y1 = last_cell(x.y + reach, g.inv_h, y0);
+        const int z0 = cell_of(x.z - reach, g.inv_h), z1 = last_cell(x.z + reach, g.inv_h, z0);
         // tests candidate j exactly
         auto consider = [&](int j) {
             const V3 xj = ld3(xq, j);

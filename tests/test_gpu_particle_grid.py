@@ -141,3 +141,11 @@ def test_own_radius_beyond_the_maximum(cuda):
     want = op.step(model._host, particles.params(model), q, qd, None, none, 1.0 / 240.0, 1, 0.9, False)[0][0]
     assert solver._particles.status() == 0 and not np.array_equal(want, q[0])
     assert np.array_equal(b.particle_q[0].cpu().numpy().view(np.uint32), want.astype(np.float32).view(np.uint32))
+
+
+@pytest.mark.parametrize("axis,far", [(0, 1.0e9), (1, 1.0e9), (2, 1.0e9), (0, -1.0e9), (2, -3.0e38)])
+def test_cells_beyond_an_int(cuda, axis, far):
+    # one coordinate's cell is the largest or smallest int; the particles touch in the other two
+    p = np.random.default_rng(6).uniform(-0.06, 0.06, (24, 3))
+    p[:, axis] = far
+    _compare(_rows([(row, 0.015) for row in p], cuda), iterations=2)
