@@ -85,8 +85,9 @@ def group_share_words(group_threads: int, arena_words: int = ARENA_WORDS_TWO_CTA
     return (arena_words // (CTA_THREADS // group_threads)) & ~1
 
 
-def default_mode(max_world_bodies: int, world_count: int, sms: int | None = None) -> tuple:
-    """(mode, group_threads) of the step for `world_count` worlds of at most `max_world_bodies` bodies.
+def default_mode(max_world_bodies: int, world_count: int | None = None, sms: int | None = None) -> tuple:
+    """(mode, group_threads) of the step for `world_count` worlds of at most `max_world_bodies` bodies; without
+    a world count the smallest group that holds the largest world.
 
     The kernel is bound by each world's chain of dependent instructions, which a wider group shortens,
     until the worlds no longer run all at once (2 CTAs of 256 threads per SM, so 2, 4, 8, 16 groups of
@@ -106,18 +107,20 @@ def default_mode(max_world_bodies: int, world_count: int, sms: int | None = None
 
     Within the group modes the full slab is taken where it fits a group's share, else the compact one
     (they differ by a few percent); 256 threads and worlds beyond every share run as batches."""
-    sms = sms or _sm_count()
-    if world_count <= 2 * sms:
-        return "batch", 256
-    for g in (128, 64, 32):
-        slots = sms * 2 * (CTA_THREADS // g)
-        if g == 64 and max_world_bodies > 64:
-            slots *= 2
-        if world_count <= slots or g == 32:
-            for words, mode in ((SLAB_WORDS_PER_BODY, "groups"), (SLAB_WORDS_COMPACT, "groups_compact")):
-                if words * max_world_bodies <= group_share_words(g):
-                    return mode, g
-    # more worlds than fit at once, too large for one warp's share: the smallest group that holds them
+    if world_count is not None:
+        sms = sms or _sm_count()
+        if world_count <= 2 * sms:
+            return "batch", 256
+        for g in (128, 64, 32):
+            slots = sms * 2 * (CTA_THREADS // g)
+            if g == 64 and max_world_bodies > 64:
+                slots *= 2
+            if world_count <= slots or g == 32:
+                for words, mode in ((SLAB_WORDS_PER_BODY, "groups"), (SLAB_WORDS_COMPACT, "groups_compact")):
+                    if words * max_world_bodies <= group_share_words(g):
+                        return mode, g
+    # no count, or more worlds than fit at once and too large for one warp's share: the smallest group that
+    # holds them
     for g in GROUP_MODE_SIZES:
         for words, mode in ((SLAB_WORDS_PER_BODY, "groups"), (SLAB_WORDS_COMPACT, "groups_compact")):
             if words * max_world_bodies <= group_share_words(g):
