@@ -1022,8 +1022,8 @@ __global__ void __launch_bounds__(1024) world_scan_kernel(int W, int32_t* __rest
 }
 
 // Dense public Contacts arrays ordered by (world, key), and the same contacts
-// as solver records (rec), contiguous per world; one CTA per world.  Each warp
-// scans the contact counts of 32 candidates, the warps' totals give every warp
+// as solver records (rec), contiguous per world; a CTA or a warp (kWarps 8 or
+// 1, publish_by_warps below) per world.  Each warp scans the contact counts of 32 candidates, the warps' totals give every warp
 // its first output, then a warp's lanes take its outputs in order (lane k
 // writes output k, k + 32, ...), each finding its candidate by a binary search
 // of the scanned counts, so consecutive lanes store to consecutive rows of
@@ -1032,11 +1032,13 @@ __global__ void __launch_bounds__(1024) world_scan_kernel(int W, int32_t* __rest
 // 4096 worlds (180 MB), 11 / - / - / 4 us for one.
 constexpr int kPubT = 256;
 
+template <int kWarps>
 __global__ void __launch_bounds__(kPubT) publish_kernel(NbModelDesc m, NbContactSeg seg, NbContactsPublic pub) {
-    constexpr int kWarps = kPubT / 32;
+    constexpr int kWorlds = kPubT / (32 * kWarps);  // worlds per CTA
+    static_assert(kWarps == 1 || kWorlds == 1, "the warps of a world share the CTA's barrier");
     __shared__ int s_tot[2][kWarps];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int w = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % kWarps;
+    const int w = blockIdx.x * kWorlds + (threadIdx.x >> 5) / kWarps;
     if (w >= m.world_count) return;
     const float4* slots = reinterpret_cast<const float4*>(seg.slots);
     float4* rec = reinterpret_cast<float4*>(seg.rec);
@@ -1062,16 +1064,20 @@ __global__ void __launch_bounds__(kPubT) publish_kernel(NbModelDesc m, NbContact
         }
         const int tot = __shfl_sync(kFull, x, 31);
         int64_t at = dst0 + running;
-        // the totals of two rounds alternate, so one barrier per round is enough
-        if (lane == 0) s_tot[round & 1][warp] = tot;
-        __syncthreads();
+        if constexpr (kWarps == 1) {
+            running += tot;
+        } else {
+            // the totals of two rounds alternate, so one barrier per round is enough
+            if (lane == 0) s_tot[round & 1][warp] = tot;
+            __syncthreads();
 #pragma unroll
-        for (int k = 0; k < kWarps; ++k) {
-            const int v = s_tot[round & 1][k];
-            if (k < warp) at += v;
-            running += v;
+            for (int k = 0; k < kWarps; ++k) {
+                const int v = s_tot[round & 1][k];
+                if (k < warp) at += v;
+                running += v;
+            }
+            ++round;
         }
-        ++round;
         for (int o0 = 0; o0 < tot; o0 += 32) {
             const int o = o0 + lane;
             // source lane: the number of lanes whose inclusive sum is <= o
@@ -1301,6 +1307,21 @@ cudaError_t narrow_occupancy(NarrowOccupancy* out) {
 // mixed worlds (two substeps) 652 / 668, 4096 mixed worlds (one collide) 566 / 510.
 bool narrow_is_small(const NbModelDesc* m, int sms) { return m->body_count <= sms * kGjkBlocksFew * kNT; }
 
+// Whether worlds are published by a warp each, in place of a CTA.  Up to 32 pairs a warp takes a world's counts
+// in one round, and seven warps of a CTA would idle; larger worlds want the CTA's rounds side by side until the
+// CTAs come in so many waves (8 at once per SM) that fewer of them are worth more rounds.  us, warp / CTA:
+//     pairs per world     1184 worlds     2368 worlds     4736 worlds     18944 worlds
+//                  11       5.9 /  7.7      7.0 / 11.2      9.6 / 18.4      26.8 / 61.8
+//                 136       7.4 /  8.2      9.1 / 12.4     13.1 / 20.1      46.9 / 91.8
+//                 240       8.9 /  8.6     10.6 / 12.4     14.8 / 20.7
+//                 820      10.9 /  9.7     15.8 / 15.9     27.4 / 35.2
+//                3000      19.2 / 14.3     31.5 / 25.9     52.2 / 51.8
+bool publish_by_warps(const NbModelDesc* m, int sms) {
+    const long long pairs = m->pair_count, worlds = m->world_count;
+    return pairs <= 32 * worlds || (worlds > 8LL * sms && pairs <= 256 * worlds) ||
+           (worlds > 16LL * sms && pairs <= 1024 * worlds);
+}
+
 }  // namespace
 
 cudaError_t nb_launch_collide(const NbModelDesc* m, const float* body_q, const NbContactSeg* seg, int grid,
@@ -1346,7 +1367,8 @@ cudaError_t nb_launch_publish(const NbModelDesc* m, const NbContactSeg* seg, con
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int worlds = m->world_count < 1 ? 1 : m->world_count;
-    publish_kernel<<<worlds, kPubT, 0, stream>>>(*m, *seg, *pub);
+    if (publish_by_warps(m, sm_count())) publish_kernel<1><<<(worlds + 7) / 8, kPubT, 0, stream>>>(*m, *seg, *pub);
+    else publish_kernel<kPubT / 32><<<worlds, kPubT, 0, stream>>>(*m, *seg, *pub);
     return cudaGetLastError();
 }
 
