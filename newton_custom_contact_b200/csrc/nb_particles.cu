@@ -680,11 +680,6 @@ NB_D M33 from_cols(V3 a, V3 b, V3 c) {
 }
 NB_D V3 col(const M33& m, int c) { return V3{m.m[0][c], m.m[1][c], m.m[2][c]}; }
 
-// Lanes that share one particle's elements in particle_bending_kernel: an inner cloth particle has 4
-// bending edges, so each lane computes one, and the lanes then add all of them in ascending element index.
-constexpr int kElemGroup = 4;
-constexpr int kElemSlots = kThreads / kElemGroup;  // particles per block
-
 // One lane's terms: up to 4 vertices' corrections grad * mag (bit r of `on` when vertex r is the
 // particle and the term is live).
 struct ElemTerms {
@@ -693,17 +688,25 @@ struct ElemTerms {
     unsigned on;
 };
 
-// The lanes' terms added to every lane's delta, lane after lane, vertex after vertex.
+// The terms of the group's first `lanes` lanes added to every lane's delta, lane after lane, vertex after
+// vertex.
+template <int kLanes>
 NB_D V3 add_terms(const ElemTerms& t, unsigned gmask, int lanes, V3 delta) {
-    for (int k = 0; k < lanes; ++k) {
-        const unsigned on = __shfl_sync(gmask, t.on, k, kElemGroup);
+    if constexpr (kLanes == 1) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            if (!((on >> r) & 1u)) continue;
-            const V3 gr = V3{__shfl_sync(gmask, t.grad[r].x, k, kElemGroup),
-                             __shfl_sync(gmask, t.grad[r].y, k, kElemGroup),
-                             __shfl_sync(gmask, t.grad[r].z, k, kElemGroup)};
-            delta = add(delta, mul(gr, __shfl_sync(gmask, t.mag[r], k, kElemGroup)));
+        for (int r = 0; r < 4; ++r)
+            if ((t.on >> r) & 1u) delta = add(delta, mul(t.grad[r], t.mag[r]));
+    } else {
+        for (int k = 0; k < lanes; ++k) {
+            const unsigned on = __shfl_sync(gmask, t.on, k, kLanes);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (!((on >> r) & 1u)) continue;
+                const V3 gr = V3{__shfl_sync(gmask, t.grad[r].x, k, kLanes),
+                                 __shfl_sync(gmask, t.grad[r].y, k, kLanes),
+                                 __shfl_sync(gmask, t.grad[r].z, k, kLanes)};
+                delta = add(delta, mul(gr, __shfl_sync(gmask, t.mag[r], k, kLanes)));
+            }
         }
     }
     return delta;
@@ -749,11 +752,10 @@ NB_D void edge_terms(const NbParticleDesc& pd, const float* xq, const float* vq,
     }
 }
 
-// One term of a tetrahedron (solve_tetrahedra, kernels.py:459-628) as seen by particle i: term 0 the
-// stretch (trace(F^T F) - 3), term 1 the volume (det F - 1), each a compliant constraint with compliance
-// `relaxation` (the solver's soft_body_relaxation) scaled by the inverse rest volume.
-NB_D void tet_term(const NbParticleDesc& pd, const float* xq, int i, int e, int term, float dt, ElemTerms& t) {
-    t.on = 0u;
+// The two terms of a tetrahedron (solve_tetrahedra, kernels.py:459-628) as seen by particle i, added to its
+// delta: the stretch (trace(F^T F) - 3), then the volume (det F - 1), each a compliant constraint with
+// compliance `relaxation` (the solver's soft_body_relaxation) scaled by the inverse rest volume.
+NB_D V3 tet_terms(const NbParticleDesc& pd, const float* xq, int i, int e, float dt, V3 delta) {
     const int* ix = pd.tet_indices + 4 * e;
     const V3 x0 = ld3(xq, ix[0]), x1 = ld3(xq, ix[1]), x2 = ld3(xq, ix[2]), x3 = ld3(xq, ix[3]);
     const float w[4] = {pd.particle_inv_mass[ix[0]], pd.particle_inv_mass[ix[1]], pd.particle_inv_mass[ix[2]],
@@ -768,65 +770,67 @@ NB_D void tet_term(const NbParticleDesc& pd, const float* xq, int i, int e, int 
     const M33 Fm = matmul3(Ds, Dm);
     const V3 f1 = col(Fm, 0), f2 = col(Fm, 1), f3 = col(Fm, 2);
     const float tr = dot(f1, f1) + dot(f2, f2) + dot(f3, f3);
-    float C;
-    M33 dC;
-    if (term == 0) {
-        C = tr - 3.0f;
-        for (int r = 0; r < 3; ++r)
-            for (int c = 0; c < 3; ++c) dC.m[r][c] = Fm.m[r][c] * 2.0f;
-    } else {
-        C = det3(Fm) - 1.0f;
-        dC = from_cols(cross(f2, f3), cross(f3, f1), cross(f1, f2));
+    for (int term = 0; term < 2; ++term) {
+        float C;
+        M33 dC;
+        if (term == 0) {
+            C = tr - 3.0f;
+            for (int r = 0; r < 3; ++r)
+                for (int c = 0; c < 3; ++c) dC.m[r][c] = Fm.m[r][c] * 2.0f;
+        } else {
+            C = det3(Fm) - 1.0f;
+            dC = from_cols(cross(f2, f3), cross(f3, f1), cross(f1, f2));
+        }
+        if (C == 0.0f) continue;
+        const M33 dP = matmul3(dC, inv_QT);
+        V3 grad[4];
+        grad[1] = col(dP, 0);
+        grad[2] = col(dP, 1);
+        grad[3] = col(dP, 2);
+        grad[0] = sub(sub(neg(grad[1]), grad[2]), grad[3]);
+        const float wsum = dot(grad[0], grad[0]) * w[0] + dot(grad[1], grad[1]) * w[1] +
+                           dot(grad[2], grad[2]) * w[2] + dot(grad[3], grad[3]) * w[3];
+        if (!(wsum > 0.0f)) continue;
+        float alpha = pd.soft_body_relaxation / dt / dt;
+        if (inv_rest_volume > 0.0f) alpha *= inv_rest_volume;
+        const float dlambda = -C / (wsum + alpha);
+        for (int r = 0; r < 4; ++r)
+            if (ix[r] == i) delta = add(delta, mul(grad[r], w[r] * dlambda));
     }
-    if (C == 0.0f) return;
-    const M33 dP = matmul3(dC, inv_QT);
-    V3* grad = t.grad;
-    grad[1] = col(dP, 0);
-    grad[2] = col(dP, 1);
-    grad[3] = col(dP, 2);
-    grad[0] = sub(sub(neg(grad[1]), grad[2]), grad[3]);
-    const float wsum = dot(grad[0], grad[0]) * w[0] + dot(grad[1], grad[1]) * w[1] + dot(grad[2], grad[2]) * w[2] +
-                       dot(grad[3], grad[3]) * w[3];
-    if (!(wsum > 0.0f)) return;
-    float alpha = pd.soft_body_relaxation / dt / dt;
-    if (inv_rest_volume > 0.0f) alpha *= inv_rest_volume;
-    const float dlambda = -C / (wsum + alpha);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        t.mag[r] = w[r] * dlambda;
-        if (ix[r] == i) t.on |= 1u << r;
-    }
+    return delta;
 }
 
 // Bending edges, then tetrahedra, of one particle, added to its delta after the constraint kernel's terms
-// (the same order as one sequential sum): kElemGroup lanes per particle compute one element (one term of a
-// tetrahedron) each.  A kernel of its own so that the constraint kernel keeps its register budget.  The
-// solver zeroes the multipliers every iteration.
+// (the same order as one sequential sum).  A kernel of its own so that the constraint kernel keeps its
+// register budget.  The solver zeroes the multipliers every iteration.  kLanes lanes serve one particle: an
+// inner cloth particle has 4 bending edges, so with 4 each lane computes one, and the lanes then add all of
+// them in ascending index; tetrahedra, whose two terms share most of their work, take one lane.  Which form
+// runs: elements_by_lanes below.
+template <int kLanes>
 __global__ void __launch_bounds__(kThreads) particle_bending_kernel(NbParticleDesc pd, NbParticleIO io, float dt) {
-    const int lane = threadIdx.x & (kElemGroup - 1);
-    const unsigned gmask = ((1u << kElemGroup) - 1u) << (threadIdx.x & 31 & ~(kElemGroup - 1));
-    const int i = blockIdx.x * kElemSlots + threadIdx.x / kElemGroup;
+    const int lane = threadIdx.x & (kLanes - 1);
+    const unsigned gmask = ((1u << kLanes) - 1u) << (threadIdx.x & 31 & ~(kLanes - 1));
+    const int i = blockIdx.x * (kThreads / kLanes) + threadIdx.x / kLanes;
     if (i >= pd.particle_count) return;
     const int e_lo = pd.edge_count > 0 ? pd.particle_edge_start[i] : 0;
     const int e_hi = pd.edge_count > 0 ? pd.particle_edge_start[i + 1] : 0;
-    const int t_lo = pd.tet_count > 0 ? pd.particle_tet_start[i] : 0;
-    const int t_hi = pd.tet_count > 0 ? pd.particle_tet_start[i + 1] : 0;
+    int t_lo = 0, t_hi = 0;
+    if (kLanes == 1 && pd.tet_count > 0) {
+        t_lo = pd.particle_tet_start[i];
+        t_hi = pd.particle_tet_start[i + 1];
+    }
     if (e_lo == e_hi && t_lo == t_hi) return;
     const float* xq = io.particle_q_out;
     const float* vq = io.particle_qd_out;
     V3 delta = ld3(io.delta, i);
     ElemTerms t;
-    for (int k = e_lo; k < e_hi; k += kElemGroup) {
+    for (int k = e_lo; k < e_hi; k += kLanes) {
         t.on = 0u;
         if (k + lane < e_hi) edge_terms(pd, xq, vq, i, pd.particle_edge_list[k + lane], dt, t);
-        delta = add_terms(t, gmask, min(e_hi - k, kElemGroup), delta);
+        delta = add_terms<kLanes>(t, gmask, min(e_hi - k, kLanes), delta);
     }
-    // two terms per tetrahedron: lane 2 a + term takes a term of the a-th
-    for (int k = 2 * t_lo; k < 2 * t_hi; k += kElemGroup) {
-        t.on = 0u;
-        if (k + lane < 2 * t_hi) tet_term(pd, xq, i, pd.particle_tet_list[(k + lane) >> 1], (k + lane) & 1, dt, t);
-        delta = add_terms(t, gmask, min(2 * t_hi - k, kElemGroup), delta);
-    }
+    if constexpr (kLanes == 1)
+        for (int k = t_lo; k < t_hi; ++k) delta = tet_terms(pd, xq, i, pd.particle_tet_list[k], dt, delta);
     if (lane == 0) st3(io.delta, i, delta);
 }
 
@@ -1003,6 +1007,28 @@ cudaError_t grid_layout(Grid& g, const NbParticleIO* io, int P, cudaStream_t st)
     return cudaMemsetAsync(g.count, 0, sizeof(int32_t) * (size_t)M, st);
 }
 
+// Whether a particle's bending edges get 4 lanes.  They shorten its chain, but repeat its loads and sums: worth
+// it while the blocks with edges (about one particle per edge, 64 to a block) run all at once, 2 per SM, and the
+// blocks without do not count.  us per substep of 4 iterations (148 SMs), 4 lanes / 1: sheets of 3,604 / 10,004 /
+// 16,904 / 19,604 / 40,004 particles 45 / 58, 57 / 70, 64 / 76, 80 / 78, 125 / 110; a sheet of 10,000 beside
+// 100,000 / 200,000 / 300,000 loose particles 408 / 422, 715 / 718, 965 / 964.  Tetrahedra share most of their
+// two terms' work in one lane: blocks of 125 / 4,096 / 29,791 particles, the terms on lanes of their own 147 /
+// 180 / 349, in one 107 / 181 / 237.
+bool elements_by_lanes(const NbParticleDesc& pd) {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long wave = 2LL * sms * (kThreads / 4);
+    return pd.tet_count == 0 && pd.edge_count <= wave && pd.particle_count <= 12 * wave;
+}
+
+void launch_bending(const NbParticleDesc& pd, const NbParticleIO& io, float dt, cudaStream_t st) {
+    const int P = pd.particle_count;
+    if (elements_by_lanes(pd))
+        particle_bending_kernel<4><<<(P + kThreads / 4 - 1) / (kThreads / 4), kThreads, 0, st>>>(pd, io, dt);
+    else
+        particle_bending_kernel<1><<<(P + kThreads - 1) / kThreads, kThreads, 0, st>>>(pd, io, dt);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1068,7 +1094,7 @@ int nb_particle_step(const NbParticleDesc* pd, const NbParticleIO* io, const NbS
                                                                                 g, table);
         }
         if (pd->edge_count > 0 || pd->tet_count > 0)
-            particle_bending_kernel<<<(P + kElemSlots - 1) / kElemSlots, kThreads, 0, st>>>(*pd, *io, dt);
+            launch_bending(*pd, *io, dt, st);
         if (g.small && it + 1 < iterations)
             particle_regrid_kernel<<<1, 1024, 0, st>>>(*pd, *io, dt, g, 1);
         else

@@ -195,3 +195,36 @@ def test_tetrahedral_block_bit_exact(cuda):
     assert np.array_equal(_bits(s.particle_q.cpu().numpy()), _bits(q))
     assert np.array_equal(_bits(s.particle_qd.cpu().numpy()), _bits(qd))
     assert float(q[:, 2].min()) < 0.02  # it reached the ground
+
+
+@pytest.mark.parametrize("tets", [False, True])
+def test_bending_edges_with_and_without_tetrahedra(cuda, tets):
+    """A tilted sheet dropped on the ground, its bending edges by 4 lanes per particle; with tetrahedra on some of
+    its particles, both by one."""
+    from newton_custom_contact_b200 import ModelBuilder
+
+    rng = np.random.default_rng(5)
+    b = ModelBuilder()
+    b.add_ground_plane()
+    n, h = 7, 0.05
+    idx = {(i, j): b.add_particle((i * h, j * h, 0.03 + 0.02 * i + rng.uniform(0.0, 0.01)), (0.0, 0.0, -0.5), 0.02,
+                                  radius=0.01) for i in range(n) for j in range(n)}
+    for i in range(n - 1):
+        for j in range(n - 1):
+            b.add_edge(idx[i + 1, j], idx[i, j + 1], idx[i, j], idx[i + 1, j + 1], edge_ke=20.0, edge_kd=0.1)
+            if tets and (i + j) % 3 == 0:
+                top = b.add_particle((i * h + 0.02, j * h + 0.02, 0.09 + 0.02 * i), (0.0, 0.0, -0.5), 0.02, radius=0.01)
+                a, c, d = idx[i, j], idx[i + 1, j], idx[i, j + 1]
+                if b.add_tetrahedron(a, c, d, top, 1e3, 1e3) <= 0:
+                    b.add_tetrahedron(a, d, c, top, 1e3, 1e3)
+    model = b.finalize(device=cuda)
+    assert model.edge_count > 0 and (model.tet_count > 0) == tets
+    s, solver, pipe = _gpu_run(model, 24)
+    q, qd = model.host("particle_q").copy(), model.host("particle_qd").copy()
+    for _ in range(24):
+        soft = op.soft_collide(model._host, q, None, pipe.soft_contact_margin, pipe.soft_contact_max)
+        q, qd = op.step(model._host, particles.params(model), q, qd, None, soft, DT, ITERS, 0.9,
+                        soft_body_relaxation=solver.soft_body_relaxation)
+    assert np.isfinite(q).all() and solver._particles.status() == 0
+    assert np.array_equal(_bits(s.particle_q.cpu().numpy()), _bits(q))
+    assert np.array_equal(_bits(s.particle_qd.cpu().numpy()), _bits(qd))
