@@ -247,7 +247,7 @@ struct Grid {
 };
 
 constexpr int kRangeBuckets = 1024;  // buckets whose ranges one block lays out contiguously
-constexpr int kSmallParticles = 4096;  // most particles (and buckets) one block rebuilds the grid of
+constexpr int kSmallParticles = 3072;  // most particles (and buckets) one block rebuilds the grid of
 constexpr int kMinSorted = 8;        // fewest buckets of the sorted form: a row of 5 cells never wraps onto itself
 
 NB_D int cell_of(float x, float inv_h) { return (int)floorf(x * inv_h); }
@@ -858,9 +858,11 @@ __global__ void __launch_bounds__(kThreads) particle_apply_kernel(NbParticleDesc
 }
 
 // One block applies the deltas (`apply`; the first grid of a substep has none yet) and rebuilds the whole
-// grid: counts in shared memory, their scan, ranges and entries.  Up to kSmallParticles the three kernels
-// this replaces (apply, ranges, scatter) are launch and load latency: 3,010 particles, 4 iterations, 149 ->
-// 140 us per substep.
+// grid: counts in shared memory, their scan, ranges and entries.  It saves two launches of the three kernels it
+// replaces (apply, ranges, scatter), and its one SM's work grows with the particles where theirs is latency.
+// us per substep of 4 iterations, one block / three kernels, launched one by one: 1,902 particles 114 / 130,
+// 2,560 122 / 132, 3,072 123 / 132, 3,584 132 / 133, 4,096 131 / 131; replayed from a captured graph, where
+// launches cost less: 88 / 92, 96 / 91, 101 / 94, 106 / 94, 108 / 88.  The line is between the two crossings.
 __global__ void __launch_bounds__(1024) particle_regrid_kernel(NbParticleDesc pd, NbParticleIO io, float dt, Grid g,
                                                                int apply) {
     constexpr int kT = 1024, kPer = kSmallParticles / kT;

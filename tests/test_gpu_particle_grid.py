@@ -149,3 +149,8 @@ def test_cells_beyond_an_int(cuda, axis, far):
     p = np.random.default_rng(6).uniform(-0.06, 0.06, (24, 3))
     p[:, axis] = far
     _compare(_rows([(row, 0.015) for row in p], cuda), iterations=2)
+
+
+@pytest.mark.parametrize("count", [2047, 2048, 2049, 3071, 3072, 3073])
+def test_counts_at_the_border_of_one_block(cuda, count):
+    _compare(_cloud(count, 0.5 * 0.026 * count ** (1.0 / 3.0), (0.1, -0.2, 0.3), count, cuda=cuda))
