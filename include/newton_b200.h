@@ -651,9 +651,9 @@ typedef struct NbParticleIO {
     float* particle_q_out;     /* [P,3] state_out positions */
     float* particle_qd_out;    /* [P,3] state_out velocities */
     float* delta;              /* [P,3] scratch: the iteration's position corrections */
-    int32_t* grid_head;        /* [2*grid_size] scratch: the cell grid's bucket ranges and entries (or its bucket lists) */
-    int32_t* grid_next;        /* [P] scratch: the cell grid's bucket counts (or list links) */
-    int32_t grid_size;         /* a power of two; 2 P and more hold the faster, sorted form of the grid */
+    int32_t* grid_head;        /* [2*grid_size] scratch: the cell grid's entries and buckets (or its bucket lists) */
+    int32_t* grid_next;        /* [P] scratch: the cell grid's bucket counts where they fit (or list links) */
+    int32_t grid_size;         /* a power of two; from 2 P on it holds the faster, sorted form of the grid (P > 8) */
     int32_t enable_restitution; /* 1: apply_particle_shape_restitution (kernels.py:34-112) after the iterations */
     uint32_t* status;          /* [1] NB_STATUS_* bits (sticky, cleared by the caller) */
 } NbParticleIO;

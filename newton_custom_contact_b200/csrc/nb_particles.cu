@@ -227,17 +227,20 @@ __global__ void __launch_bounds__(kScanThreads) soft_write_kernel(NbParticleDesc
 // Neighbour search.  Cells have the size of the largest contact distance; a cell's bucket is
 // (cx + cy K1 + cz K2) mod M, so cells that follow each other in x are buckets that follow each other,
 // and the up to 3 cells of one (cy, cz) row around a particle are one run of the particles in bucket
-// order: 9 runs of about 14 particles in place of 27 chains.  Two forms:
+// order: 9 runs in place of 27 chains.  Two forms:
 //   sorted: per iteration the particles are counted into the buckets (integrate / apply), the buckets
 //           get their ranges (particle_ranges_kernel) and the particles' entries are written there
 //           (particle_scatter_kernel).  An entry is 8 bytes: the position within 4 cells, 10 bits per
-//           axis, and the particle -- enough to reject five of six candidates with one load.
+//           axis, and the particle -- enough to reject most candidates with one load.  Up to 2 P buckets:
+//           most candidates of a scattered particle are strangers that share a bucket with its cells, and
+//           half as many buckets have twice as many of them (us per substep of 4 iterations, up to P / up to
+//           2 P buckets: 100,000 scattered particles 245 / 210, piled ones 276 / 260).
 //   lists:  linked lists per bucket (head / next), for scratch too small for the sorted form.
 struct Grid {
     int32_t* head;   // lists: [2][M] first particle of a bucket, -1 empty
     int32_t* next;   // lists: [P] next particle of the same bucket
-    int2* range;     // sorted: [M] first and last + 1 entry of a bucket
     int2* entry;     // sorted: [P] (packed position, particle) in bucket order
+    int32_t* first;  // sorted: first entries of the buckets and the blocks' ends (bucket_at)
     int32_t* count;  // sorted: [M] particles of a bucket; all zero outside counting .. scatter
     int32_t* cursor; // sorted: [1] entries handed out so far; the active particles once all are
     uint32_t mask;   // M - 1
@@ -247,9 +250,13 @@ struct Grid {
 };
 
 constexpr int kRangeBuckets = 1024;  // buckets whose ranges one block lays out contiguously
-constexpr int kSmallParticles = 3072;  // most particles (and buckets) one block rebuilds the grid of
+constexpr int kSmallParticles = 3072;  // most particles one block rebuilds the grid of
+constexpr int kSmallBuckets = 4096;     // their buckets: fewer than twice as many, a power of two
 constexpr int kMinSorted = 8;        // fewest buckets of the sorted form: a row of 5 cells never wraps onto itself
 
+// place of bucket b's first entry; the place behind it holds its end, which is the next bucket's first entry or
+// the end of the block
+__host__ __device__ __forceinline__ uint32_t bucket_at(uint32_t b) { return b + b / kRangeBuckets; }
 NB_D int cell_of(float x, float inv_h) { return (int)floorf(x * inv_h); }
 // the last of the cells searched from `first` on: at most 5, which keeps the loops bounded whatever the
 // scale, and none past the largest int, where far positions end up
@@ -317,8 +324,10 @@ __global__ void __launch_bounds__(kThreads) particle_ranges_kernel(Grid g) {
     int at = s_base + s_warp[warp] + x - sum;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-        if (b0 + k <= g.mask) g.range[b0 + k] = make_int2(at, at + c[k]);
+        const uint32_t b = b0 + k;
+        if (b <= g.mask) g.first[bucket_at(b)] = at;
         at += c[k];
+        if (b == g.mask || (b < g.mask && b % kRangeBuckets == kRangeBuckets - 1)) g.first[bucket_at(b) + 1] = at;
     }
 }
 
@@ -328,7 +337,7 @@ __global__ void __launch_bounds__(kThreads) particle_scatter_kernel(NbParticleDe
     if (p >= pd.particle_count || !active(pd, p)) return;
     const V3 x = ld3(xq, p);
     const uint32_t b = cell_hash(cell_of(x.x, g.inv_h), cell_of(x.y, g.inv_h), cell_of(x.z, g.inv_h), g.mask);
-    const int at = g.range[b].x + atomicSub(&g.count[b], 1) - 1;
+    const int at = g.first[bucket_at(b)] + atomicSub(&g.count[b], 1) - 1;
     g.entry[at] = make_int2((int)entry_word(pd, p, x, g.inv_h), p);
 }
 
@@ -370,10 +379,12 @@ __global__ void __launch_bounds__(kThreads) particle_integrate_kernel(NbParticle
 // Bound by the latency of the dependent loads and, at size, by instructions, so the steps are few and
 // wide: one row lookup per lane, candidates in runs of 32, all arrays of a kept candidate at once; the
 // sorted form takes the particles in bucket order, so that a block's particles share their candidates in
-// L1.  Measured at 110,002 particles (54 candidates, 4 contacts each on average; 8 iterations, per
-// substep) with 4 / 8 / 16 / 32 lanes: 1369 / 990 / 967 / 1440 us; at 3,010 particles (4 iterations):
-// 286 / 205 / 150 / 147 us.  Linked lists of the cells, whose candidates are one dependent load after
-// another, with one lane sorting and summing for its group of 8, took 2215 and 240 us.
+// L1.  Measured at 110,002 particles (4 contacts each on average; 8 iterations, per substep) with 4 / 8 / 16 /
+// 32 lanes and up to P buckets: 1369 / 990 / 967 / 1440 us; at 3,010 particles (4 iterations): 286 / 205 / 150 /
+// 147 us; now, with 16 lanes and up to 2 P buckets, 953 and 136 us.  Linked lists of the cells, whose candidates
+// are one dependent load after another, with one lane sorting and summing for its group of 8, took 2215 and
+// 240 us; they stay faster by 1.15 to 1.3 times where hardly any particles meet (20,000 scattered ones 120
+// against 156 us per substep of 8 iterations, 100,000 368 against 426), for they need two kernels less.
 constexpr int kGroup = 16;                 // lanes per particle
 constexpr int kSlots = kThreads / kGroup;  // particles per block
 constexpr int kAhead = 2;                  // candidate loads a lane has in flight
@@ -472,12 +483,12 @@ particle_constraints_kernel(NbParticleDesc pd, NbParticleIO io, NbSoftContacts s
                     key = (((uint32_t)cy & 3u) << 18) | (((uint32_t)cz & 3u) << 28);
                     const uint32_t b = cell_hash(x0, cy, cz, g.mask);
                     const uint32_t e = b + (uint32_t)(x1 - x0), cut = b | bm;
-                    beg = g.range[b].x;
-                    len = g.range[min(e, cut)].y - beg;
+                    beg = g.first[bucket_at(b)];
+                    len = g.first[bucket_at(min(e, cut)) + 1] - beg;
                     tot = len;
                     if (e > cut) {
-                        beg2 = g.range[(cut + 1u) & g.mask].x;
-                        tot += g.range[e & g.mask].y - beg2;
+                        beg2 = g.first[bucket_at((cut + 1u) & g.mask)];
+                        tot += g.first[bucket_at(e & g.mask) + 1] - beg2;
                     }
                 }
                 int run = tot;
@@ -865,8 +876,8 @@ __global__ void __launch_bounds__(kThreads) particle_apply_kernel(NbParticleDesc
 // launches cost less: 88 / 92, 96 / 91, 101 / 94, 106 / 94, 108 / 88.  The line is between the two crossings.
 __global__ void __launch_bounds__(1024) particle_regrid_kernel(NbParticleDesc pd, NbParticleIO io, float dt, Grid g,
                                                                int apply) {
-    constexpr int kT = 1024, kPer = kSmallParticles / kT;
-    __shared__ int s_count[kSmallParticles];
+    constexpr int kT = 1024, kPer = kSmallParticles / kT, kBuckets = kSmallBuckets / kT;  // per thread
+    __shared__ int s_count[kSmallBuckets];
     __shared__ int s_warp[kT / 32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int M = (int)g.mask + 1;
@@ -885,10 +896,10 @@ __global__ void __launch_bounds__(1024) particle_regrid_kernel(NbParticleDesc pd
         rank[k] = atomicAdd(&s_count[bucket[k]], 1);
     }
     __syncthreads();
-    int c[kPer], sum = 0;
+    int c[kBuckets], sum = 0;
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-        const int b = t * kPer + k;
+    for (int k = 0; k < kBuckets; ++k) {
+        const int b = t * kBuckets + k;
         c[k] = b < M ? s_count[b] : 0;
         sum += c[k];
     }
@@ -913,11 +924,12 @@ __global__ void __launch_bounds__(1024) particle_regrid_kernel(NbParticleDesc pd
     __syncthreads();
     int at = x - sum + (warp > 0 ? s_warp[warp - 1] : 0);
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-        const int b = t * kPer + k;
+    for (int k = 0; k < kBuckets; ++k) {
+        const int b = t * kBuckets + k;
         if (b < M) {
-            g.range[b] = make_int2(at, at + c[k]);
+            g.first[bucket_at(b)] = at;
             s_count[b] = at;  // this thread alone reads and writes bucket b here
+            if (b == M - 1 || b % kRangeBuckets == kRangeBuckets - 1) g.first[bucket_at(b) + 1] = at + c[k];
         }
         at += c[k];
     }
@@ -982,16 +994,20 @@ bool check_pd(const NbParticleDesc* pd) {
     return true;
 }
 
-// Lays the neighbour search out in the caller's scratch: grid_head [2 n] and grid_next [P].  The sorted
-// form needs M <= P counts (grid_next) and M ranges + P entries (grid_head); M is the largest power of two
-// that fits, from a fourth of the particles up -- with fewer buckets its rows hold too many strangers,
-// and the lists, which use all n buckets, are taken (grid_size >= 2 P always fits).
+// Lays the neighbour search out in the caller's scratch: grid_head [2 n] and grid_next [P].  The sorted form
+// keeps its entries, buckets and cursor in grid_head, and the counts of its M buckets in grid_next where they fit
+// (M <= P), else in grid_head too.  M is the largest power of two below 2 P that fits: with about one particle
+// per bucket few strangers are met.  Below P / 4 buckets, or kMinSorted, the lists, which use all n buckets, are
+// taken.  n >= 2 P holds the sorted form for P > 8.
 cudaError_t grid_layout(Grid& g, const NbParticleIO* io, int P, cudaStream_t st) {
-    const long long room = 2LL * io->grid_size - 2;  // ints, after the cursor and up to one to align
+    const long long room = 2LL * io->grid_size - 1;  // ints, after up to one to align
+    auto ints = [&](long long M) {
+        return 2LL * P + M + (M + kRangeBuckets - 1) / kRangeBuckets + 1 + (M > P ? M : 0);
+    };
     long long M = 1;
-    while (2 * M <= P) M *= 2;
-    while (M > 1 && 2 * M + 2LL * P > room) M /= 2;
-    g.sorted = M >= kMinSorted && 4 * M >= P && 2 * M + 2LL * P <= room;
+    while (M < P) M *= 2;
+    while (M > 1 && ints(M) > room) M /= 2;
+    g.sorted = M >= kMinSorted && 4 * M >= P && ints(M) <= room;
     if (!g.sorted) {
         g.head = io->grid_head;
         g.next = io->grid_next;
@@ -999,12 +1015,12 @@ cudaError_t grid_layout(Grid& g, const NbParticleIO* io, int P, cudaStream_t st)
         return cudaMemsetAsync(g.head, 0xff, sizeof(int32_t) * (size_t)io->grid_size, st);
     }
     int32_t* base = io->grid_head + (((uintptr_t)io->grid_head & 7u) ? 1 : 0);
-    g.range = reinterpret_cast<int2*>(base);
-    g.entry = g.range + M;
-    g.cursor = base + 2 * M + 2LL * P;
-    g.count = io->grid_next;
+    g.entry = reinterpret_cast<int2*>(base);
+    g.first = base + 2LL * P;
+    g.cursor = g.first + bucket_at((uint32_t)M - 1u) + 2;
+    g.count = M > P ? g.cursor + 1 : io->grid_next;
     g.mask = (uint32_t)(M - 1);
-    g.small = P <= kSmallParticles;  // M <= P
+    g.small = P <= kSmallParticles;
     if (g.small) return cudaSuccess;
     return cudaMemsetAsync(g.count, 0, sizeof(int32_t) * (size_t)M, st);
 }

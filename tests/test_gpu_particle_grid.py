@@ -154,3 +154,20 @@ def test_cells_beyond_an_int(cuda, axis, far):
 @pytest.mark.parametrize("count", [2047, 2048, 2049, 3071, 3072, 3073])
 def test_counts_at_the_border_of_one_block(cuda, count):
     _compare(_cloud(count, 0.5 * 0.026 * count ** (1.0 / 3.0), (0.1, -0.2, 0.3), count, cuda=cuda))
+
+
+@pytest.mark.parametrize("count", [9, 1000, 5000])
+def test_scratch_off_an_eight_byte_boundary(cuda, count):
+    model = _cloud(count, 0.5 * 0.026 * count ** (1.0 / 3.0), (0.1, -0.2, 0.3), count, cuda=cuda)
+    solver = SolverXPBD(model, iterations=3)
+    ps = solver._particles
+    buf = torch.full((2 * ps.grid_size + 2,), -7, dtype=torch.int32, device=cuda)
+    ps.grid_head = buf[1:-1]
+    a, b, contacts = model.state(), model.state(), CollisionPipeline(model).contacts()
+    solver.step(a, b, contacts=contacts, control=None, dt=1.0 / 240.0)
+    q, qd = model.host("particle_q"), model.host("particle_qd")
+    none = op.soft_collide(model._host, q, None, 0.01, 0)
+    want = op.step(model._host, particles.params(model), q, qd, None, none, 1.0 / 240.0, 3, 0.9, False)[0]
+    act = (model.host("particle_flags") & 1) != 0
+    assert np.array_equal(b.particle_q.cpu().numpy()[act].view(np.uint32), want[act].astype(np.float32).view(np.uint32))
+    assert int(buf[0]) == -7 and int(buf[-1]) == -7
