@@ -116,10 +116,12 @@ __device__ __forceinline__ void ordered_flush(OrderedBatch<G>& B, int head, int 
         if (la >= 0) atomicOr(&B.own_a[t >> 5][la & (G - 1)], bit);
         if (lb >= 0) atomicOr(&B.own_b[t >> 5][lb & (G - 1)], bit);
     }
-    // Never taken (m > 0).  With a single call site the compiler merges the solve's products with the
-    // code around it and contracts other pairs of them into FMAs than in the other kernels that call it;
-    // a second site keeps one form, so that the product build's results are the same bits for every group
-    // size and from build to build.
+    // Never taken (m > 0).  With a single call site the compiler inlines the solve and contracts other pairs
+    // of its products into FMAs than in the other kernels that call it (3e-7 relative per step); with a second
+    // one the product build's plain step gives the same bits on every schedule.  That is how this compiler
+    // behaves, not a rule of the language: tests/test_gpu_schedule_bits.py compares the schedules.  The
+    // warm-started step is not covered: groups of 32 with the compact slab differ from the others by 1e-10
+    // relative.  The parity build, which contracts nothing, needs none of this.
     if (m < 0) solve(t, B.d[t]);
     ordered_sync<G, kCTA>(g);  // the rows and the marks are visible
     float acc[6];
