@@ -1047,8 +1047,8 @@ __device__ __forceinline__ void adjoint_contacts(const NbModelDesc& m, const NbX
 // One block row per chunk: a contact's chunks, each a pass over the whole contact with dual numbers, run
 // on kChunks threads at once instead of one after another.  Bound by that chain: with some 20,000 active
 // contacts one thread per contact is one warp per scheduler.  256 stacks of 16 boxes, us per launch: 46 in
-// one thread, 31 in chunks of four directions, 40 of two; 27 with three CTAs per SM (168 registers) in
-// place of two.
+// one thread, 31 in chunks of four directions, 40 of two; 27 with three CTAs per SM (168 registers, 452
+// bytes of spill stores) in place of two.
 __global__ void __launch_bounds__(kThreads, 3) adjoint_contacts_kernel(NbModelDesc m, NbXpbdParams p,
                                                                        NbAdjointIO io, NbContactSeg seg, int it,
                                                                        float dt) {

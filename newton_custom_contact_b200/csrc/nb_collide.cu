@@ -249,8 +249,8 @@ __device__ void world_by_warp(const NbModelDesc& m, const float* __restrict__ bo
 // into one contiguous run per warp; pass 1 counts each run's hits, a scan over
 // the warps gives every run its first candidate index, pass 2 writes -- the
 // candidates stay in pair order.  Pass 2 takes the hits from registers for the
-// first 8 chunks of a run (worlds of up to 8192 pairs, 128 bodies); what a
-// larger world has beyond is tested again
+// first 8 chunks of a run (worlds of up to 8192 pairs: 127 bodies over a
+// ground plane); what a larger world has beyond is tested again
 __device__ void world_by_cta(const NbModelDesc& m, const float* __restrict__ body_q, const NbContactSeg& seg, int k,
                              float4* lo, float4* hi, QueueStage& st, int* s_run, int warp, int lane) {
     const unsigned* pairs = m.pair_shapes;
@@ -842,7 +842,8 @@ gjk_prefilter_kernel(NbModelDesc m, NbContactSeg seg) {
 // never exceed the n1 <= pair_count entries the region held).
 // Latency and divergence bound: with more items than threads, resident warps
 // hide it (64 registers, 8 CTAs per SM); with fewer, each item's own chain is
-// the kernel's time, and registers without spills shorten it (128, 4 CTAs).
+// the kernel's time, and registers shorten it (128, 4 CTAs: 96 bytes of spill
+// stores; 64: 356).
 // The few-bodies variant also shares an item between two warps while there are
 // threads for that: one runs MPR, the other GJK at the same time (MPR finds no
 // overlap in 97 % or more of the items, so GJK's result is almost always used):

@@ -120,8 +120,8 @@ __device__ __forceinline__ void ordered_flush(OrderedBatch<G>& B, int head, int 
     // of its products into FMAs than in the other kernels that call it (3e-7 relative per step); with a second
     // one the product build's plain step gives the same bits on every schedule.  That is how this compiler
     // behaves, not a rule of the language: tests/test_gpu_schedule_bits.py compares the schedules.  The
-    // warm-started step is not covered: groups of 32 with the compact slab differ from the others by 1e-10
-    // relative.  The parity build, which contracts nothing, needs none of this.
+    // warm-started step is not covered: groups of 32 with the compact slab round a few values differently (4e-9
+    // relative over a step's velocities).  The parity build, which contracts nothing, needs none of this.
     if (m < 0) solve(t, B.d[t]);
     ordered_sync<G, kCTA>(g);  // the rows and the marks are visible
     float acc[6];

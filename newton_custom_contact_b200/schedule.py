@@ -91,9 +91,12 @@ def default_mode(max_world_bodies: int, world_count: int | None = None, sms: int
 
     The kernel is bound by each world's chain of dependent instructions, which a wider group shortens,
     until the worlds no longer run all at once (2 CTAs of 256 threads per SM, so 2, 4, 8, 16 groups of
-    256, 128, 64, 32 threads): the widest group that runs every world at once is taken.  Worlds of more
-    than 64 bodies keep 64 threads for as long as one warp per world would not need a second round
-    either (their body passes take three warp rounds or more); smaller ones change over at once.
+    256, 128, 64, 32 threads): the widest group that runs every world at once is taken.  (Beyond 481 bodies a
+    256-thread group's slab leaves one CTA per SM, so 149 to 296 worlds take two rounds: 296 worlds of 480 / 512
+    bodies 94 / 142 us, against 148 / 153 with groups of 128 threads and 115 / 120 with batches of 128, which
+    this rule does not choose.)  Worlds of more than 64 bodies keep 64 threads for as long as one warp per world
+    would not need a second round either (their body passes take three warp rounds or more); smaller ones change
+    over at once.
     Measured (148 SMs, 8 iterations, us per step at 256 / 128 / 64 / 32 threads; mixed shapes, 8..128 and
     8..32 bodies):
 
